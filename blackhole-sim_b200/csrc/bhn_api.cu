@@ -10,6 +10,7 @@
 
 #include <cmath>
 #include <cstdio>
+#include <mutex>
 #include <string>
 
 #include "bhn_internal.cuh"
@@ -44,6 +45,47 @@ int sm_count_current_device() {
         cached[dev] = sms;
     }
     return cached[dev];
+}
+
+// Stream-ordered allocations of the entry points that take no scratch buffer.
+// One pool per device keeps up to kPoolKeep bytes between calls (a call's
+// tables are under 10 MB); everything above that goes back to the system at the
+// next synchronisation.  The driver orders reuse across threads and streams,
+// and under stream capture the pair becomes the graph's own memory nodes.
+constexpr uint64_t kPoolKeep = 64ull << 20;
+static int device_pool(cudaMemPool_t &pool) {
+    static cudaMemPool_t pools[64] = {};
+    static std::mutex lock;
+    int dev = 0;
+    BHN_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(BHN_ERR_CUDA, "device index out of range");
+    std::lock_guard<std::mutex> g(lock);
+    if (!pools[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t p;
+        BHN_CUDA_TRY(cudaMemPoolCreate(&p, &props));
+        uint64_t keep = kPoolKeep;
+        BHN_CUDA_TRY(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+        pools[dev] = p;
+    }
+    pool = pools[dev];
+    return BHN_OK;
+}
+
+int stream_alloc(void **p, int64_t bytes, cudaStream_t s) {
+    *p = nullptr;
+    cudaMemPool_t pool;
+    int rc = device_pool(pool);
+    if (rc) return rc;
+    BHN_CUDA_TRY(cudaMallocFromPoolAsync(p, (size_t)bytes, pool, s));
+    return BHN_OK;
+}
+
+void stream_free(void *p, cudaStream_t s) {
+    if (p) cudaFreeAsync(p, s);
 }
 
 // exact helpers: bhn_exact.cuh

@@ -18,8 +18,8 @@
 //   trace_kernel     one thread per ray: continues its RK4 geodesic until it
 //                    has produced `chunk` emitting segments (or the trace
 //                    ends), appending each segment's plasma frame to a list;
-//   coef_kernel      one warp per listed segment: the synchrotron integrals
-//                    (bhn_synchrotron.cuh) at full occupancy;
+//   coef_kernel      a batch of listed segments per warp: the synchrotron
+//                    integrals (bhn_synchrotron.cuh) at full occupancy;
 //   transfer_kernel  one thread per ray: its segments' Stokes steps in order,
 //                    the optical-depth cutoff, the result when the ray ends.
 // A ray whose optical depth crosses the cutoff ends at that segment (its
@@ -274,22 +274,34 @@ __global__ void __launch_bounds__(128) grrt_trace_kernel(const TraceParams P) {
     R.trace_status = ts;
 }
 
-// One warp per listed segment (a persistent grid over this round's list).
+// The listed segments' coefficients, a batch of up to 32 per warp (a
+// persistent grid over this round's list; a short list spreads over the warps).
 __global__ void __launch_bounds__(128, 6) grrt_coef_kernel(const __grid_constant__ CoefParams P) {
     __shared__ synch::TableSmem T;
     synch::load_table(T, P.M);
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const unsigned long long n = *P.W.n_seg;
-    const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-    for (unsigned long long i = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-        const SegIn s = P.W.seg[i];
+    const int64_t n = (int64_t)*P.W.n_seg;
+    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t per = max((int64_t)1, min((int64_t)32, (n + warps - 1) / warps));
+    for (int64_t first = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per; first < n;
+         first += warps * per) {
+        const int count = (int)min(per, n - first);
+        SegIn s;
+        synch::Frame f = {0.0, 1.0, 0.0, 0.0, 0.0, 1.0};
+        if (lane < count) {
+            s = P.W.seg[first + lane];
+            f = {s.n_e, s.te, s.b, s.cos_los, s.chi, s.nu_emit};
+        }
         double c[11];
-        synch::coefficients(T, P.M, s.n_e, s.te, s.b, s.cos_los, s.chi, s.nu_emit, c);
-        double *o = P.W.coef + 12 * i;
+        synch::coefficients(T, P.M, f, count, c);
+        if (lane >= count) continue;
+        double2 *o = reinterpret_cast<double2 *>(P.W.coef + 12 * (first + lane));
 #pragma unroll
-        for (int k = 0; k < 11; ++k)
-            if (lane == k) o[k] = c[k] * (k < 4 ? s.jf : s.kf);
+        for (int k = 0; k < 11; ++k) c[k] *= k < 4 ? s.jf : s.kf;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) o[k] = make_double2(c[2 * k], c[2 * k + 1]);
+        o[5] = make_double2(c[10], 0.0);
     }
 }
 
@@ -392,11 +404,17 @@ extern "C" int bhn_grrt_render(const double *fields, const double *r_grid, int32
     if (chunk < 1)
         return fail(BHN_ERR_VALUE, "scratch too small: bhn_grrt_scratch_bytes(rays, 1) = " +
                                        std::to_string(grrt_layout(rays, 1).total) + " bytes");
-    static CoefParams C;  // ~10 KB (the model's tables): kept off the host stack; filled under the lock
-    static std::mutex lock;
-    std::lock_guard<std::mutex> g(lock);
-    int rc = synch::fill_model(model, C.M);
+    cudaStream_t s = as_stream(stream);
+    CoefParams C;
+    void *tables = nullptr;
+    // (a ray lists about a thousand segments; the same tables for every chunk, so the image does not depend on it)
+    int rc = synch::build_model(model, rays * 1000, C.M, tables, s);
     if (rc) return rc;
+    struct Free {  // the model's tables, after the last kernel below
+        void *p;
+        cudaStream_t s;
+        ~Free() { stream_free(p, s); }
+    } free_tables{tables, s};
     rc = bhn_render_prepare(view, 1, scratch, scratch_layout(1).total, stream);  // FP64 camera tables of the view
     if (rc) return rc;
     const GrrtLayout GL = grrt_layout(rays, chunk);
@@ -444,7 +462,6 @@ extern "C" int bhn_grrt_render(const double *fields, const double *r_grid, int32
     BHN_CUDA_TRY(cudaGetDevice(&dev));
     BHN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     BHN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grrt_coef_kernel, 128, 0));
-    cudaStream_t s = as_stream(stream);
     const unsigned ray_blocks = (unsigned)((rays + 127) / 128);
     const unsigned coef_blocks = (unsigned)std::min<int64_t>((rays * chunk + 3) / 4, (int64_t)sms * std::max(per_sm, 1));
     BHN_CUDA_TRY(cudaMemsetAsync(W.n_seg, 0, sizeof(unsigned long long), s));

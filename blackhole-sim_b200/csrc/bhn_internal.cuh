@@ -17,6 +17,9 @@ void set_error(const std::string &msg);
 int fail(int code, const std::string &msg);
 int cuda_fail(cudaError_t err, const char *what);
 int sm_count_current_device();
+// Stream-ordered device memory from the library's pool (BHN_OK or the error set).
+int stream_alloc(void **p, int64_t bytes, cudaStream_t s);
+void stream_free(void *p, cudaStream_t s);
 
 #define BHN_CUDA_TRY(expr)                                   \
     do {                                                     \
