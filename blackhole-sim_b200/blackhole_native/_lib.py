@@ -21,7 +21,7 @@ EXPORTED = (
     "bhn_core_version", "bhn_last_error", "bhn_device_info", "bhn_fp32_peak_probe", "bhn_fp64_peak_probe",
     "bhn_stokes_rk2_brick", "bhn_stokes_exact_brick", "bhn_sample_brick_trilinear", "bhn_sample_and_step_stokes",
     "bhn_sample_sort_scratch_bytes", "bhn_sample_and_step_stokes_sorted", "bhn_sample_brick_trilinear_sorted",
-    "bhn_sample_brick_valid_mask", "bhn_check_values",
+    "bhn_sample_points_checked", "bhn_stokes_brick_checked", "bhn_sample_brick_valid_mask", "bhn_check_values",
     "bhn_brick_tables_bytes", "bhn_brick_build_tables", "bhn_brick_pack", "bhn_brick_locate",
     "bhn_render_scratch_bytes", "bhn_render_prepare", "bhn_render_launch", "bhn_render_noalloc",
     "bhn_graph_create", "bhn_graph_launch", "bhn_graph_destroy",
@@ -122,6 +122,9 @@ def _declare(lib: ctypes.CDLL) -> None:
         "bhn_sample_brick_trilinear_sorted": ([vp, vp, i64, vp, i64, vp, i64, vp, i64, vp, vp, i64, vp], ctypes.c_int),
         "bhn_sample_and_step_stokes_sorted": ([vp, vp, i64, vp, i64, vp, i64, vp, i64, d, vp, i64, i32, vp, vp, i64,
                                                vp], ctypes.c_int),
+        "bhn_stokes_brick_checked": ([vp, i64, d, vp, i64, i32, vp, vp, vp], ctypes.c_int),
+        "bhn_sample_points_checked": ([vp, vp, i64, vp, i64, vp, i64, vp, i64, d, vp, i64, i32, vp, vp, i64, vp, vp],
+                                      ctypes.c_int),
         "bhn_sample_brick_valid_mask": ([vp, i64, vp, i64, vp, i64, vp, vp], ctypes.c_int),
         "bhn_check_values": ([vp, i64, i32, vp, vp], ctypes.c_int),
         "bhn_brick_tables_bytes": ([i32, i32, i32], i64),

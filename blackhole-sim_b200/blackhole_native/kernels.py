@@ -87,6 +87,44 @@ def _validate_sampler_device(coeffs, rg, tg, pg, points) -> int:
     return points.numel() // 3
 
 
+def _raise_grid_counts(counts) -> None:
+    """The reference's errors for the counts of bhn_sample_points_checked's three axes."""
+    for a, name in enumerate(("r", "theta", "phi")):
+        if counts[2 * a]:
+            raise ValueError(f"{name} grid must contain only finite values")
+        if counts[2 * a + 1]:
+            raise ValueError(f"{name} grid must be strictly increasing")
+
+
+def _sample_checked(c, rg, tg, pg, pts, out_width: int, ds: float = 0.0, ini=None, policy: int = 0):
+    """The sampler (or, with ``ini``, sample-and-step) on device tensors with its
+    input checks queued beside it and read back once, after it; None when the
+    sizes are wrong (the caller's checks then find the first error in the
+    reference's order)."""
+    sizes = (rg.numel(), tg.numel(), pg.numel())
+    n = pts.numel() // 3
+    if (min(sizes) < 2 or max(sizes) > 1 << 20 or c.numel() != math.prod(sizes) * COEFFS_PER_CELL or pts.numel() % 3
+            or (ini is not None and ini.numel() not in (STOKES_COMPONENTS, n * STOKES_COMPONENTS))):
+        return None
+    out = torch.empty(n * out_width, dtype=torch.float64, device=c.device)
+    L = _lib.lib()
+    scratch, sp, nbytes = _sort_scratch(n, math.prod(sizes), out.device)
+    counts = torch.empty(11, dtype=torch.int32, device=c.device)
+    _lib.check(L.bhn_sample_points_checked(dev.ptr(c), dev.ptr(rg), sizes[0], dev.ptr(tg), sizes[1], dev.ptr(pg),
+                                           sizes[2], dev.ptr(pts), n, ds, dev.ptr(ini),
+                                           0 if ini is None else ini.numel(), policy, dev.ptr(out), sp, nbytes,
+                                           dev.ptr(counts), dev.stream_ptr()))
+    k = counts.tolist()
+    _raise_grid_counts(k)
+    if k[6]:
+        raise ValueError("coeffs must contain only finite values")
+    if k[10]:
+        raise ValueError("points must contain only finite values")
+    if k[8]:
+        raise ValueError("initial must contain only finite values")
+    return out
+
+
 def _dev_f64(x, device) -> torch.Tensor:
     return x.detach().to(device=device, dtype=torch.float64).contiguous().reshape(-1)
 
@@ -120,17 +158,22 @@ def _stokes_brick(coeffs, ds_cm, initial, entry):
         c = _dev_f64(torch.as_tensor(coeffs), device)
         if c.numel() == 0 or c.numel() % COEFFS_PER_CELL:
             raise ValueError("coeffs must contain one or more flat 11-coefficient cells")
-        if dev.check_values_device(c, False)[0]:
-            raise ValueError("coeffs must contain only finite values")
         cells = c.numel() // COEFFS_PER_CELL
         ini = _dev_f64(torch.as_tensor(initial), device)
         if ini.numel() != STOKES_COMPONENTS and ini.numel() != cells * STOKES_COMPONENTS:
+            if dev.check_values_device(c, False)[0]:  # the reference's order: the coefficients come first
+                raise ValueError("coeffs must contain only finite values")
             raise ValueError("initial must contain either 4 values or 4 values per coefficient cell")
-        if dev.check_values_device(ini, False)[0]:
-            raise ValueError("initial must contain only finite values")
         out = torch.empty(cells * STOKES_COMPONENTS, dtype=torch.float64, device=device)
-        _lib.check(getattr(_lib.lib(), entry)(dev.ptr(c), cells, ds, dev.ptr(ini), ini.numel(), dev.ptr(out),
-                                              dev.stream_ptr()))
+        counts = torch.empty(2, dtype=torch.int32, device=device)
+        _lib.check(_lib.lib().bhn_stokes_brick_checked(dev.ptr(c), cells, ds, dev.ptr(ini), ini.numel(),
+                                                       int(entry == "bhn_stokes_exact_brick"), dev.ptr(out),
+                                                       dev.ptr(counts), dev.stream_ptr()))
+        bad_c, bad_s = counts.tolist()
+        if bad_c:
+            raise ValueError("coeffs must contain only finite values")
+        if bad_s:
+            raise ValueError("initial must contain only finite values")
         return out
     c = dev.host_f64(coeffs)
     if c.size == 0 or c.size % COEFFS_PER_CELL:
@@ -159,6 +202,9 @@ def sample_brick_trilinear(coeffs, r_grid, theta_grid, phi_grid, points):
     if _any_cuda(coeffs, r_grid, theta_grid, phi_grid, points):
         device = dev.require_cuda()
         c, rg, tg, pg, pts = (_dev_f64(torch.as_tensor(x), device) for x in (coeffs, r_grid, theta_grid, phi_grid, points))
+        out = _sample_checked(c, rg, tg, pg, pts, COEFFS_PER_CELL)
+        if out is not None:
+            return out
         n = _validate_sampler_device(c, rg, tg, pg, pts)
         out = torch.empty(n * COEFFS_PER_CELL, dtype=torch.float64, device=device)
         _launch_sample_trilinear(c, rg, tg, pg, pts, n, out)
@@ -187,8 +233,11 @@ def sample_and_step_stokes(coeffs, r_grid, theta_grid, phi_grid, points, ds_cm, 
     if _any_cuda(coeffs, r_grid, theta_grid, phi_grid, points, initial):
         device = dev.require_cuda()
         c, rg, tg, pg, pts = (_dev_f64(torch.as_tensor(x), device) for x in (coeffs, r_grid, theta_grid, phi_grid, points))
-        n = _validate_sampler_device(c, rg, tg, pg, pts)
         ini = _dev_f64(torch.as_tensor(initial), device)
+        out = _sample_checked(c, rg, tg, pg, pts, STOKES_COMPONENTS, ds, ini, policy)
+        if out is not None:
+            return out
+        n = _validate_sampler_device(c, rg, tg, pg, pts)
         if ini.numel() != STOKES_COMPONENTS and ini.numel() != n * STOKES_COMPONENTS:
             raise ValueError("initial must contain either 4 values or 4 values per sample point")
         if dev.check_values_device(ini, False)[0]:
@@ -213,6 +262,16 @@ def sample_and_step_stokes(coeffs, r_grid, theta_grid, phi_grid, points, ds_cm, 
 SORT_MIN_POINTS = 1 << 18   # from this many points the sampler takes them in brick-cell order
 
 
+def _sort_scratch(n: int, cells: int, device):
+    """(buffer, aligned pointer, bytes) of the cell-ordered form's scratch, or
+    (None, None, 0) for point sets taken in input order."""
+    nbytes = int(_lib.lib().bhn_sample_sort_scratch_bytes(n, cells)) if n >= SORT_MIN_POINTS else -1
+    if nbytes <= 0:
+        return None, None, 0
+    scratch = torch.empty(nbytes + 256, dtype=torch.uint8, device=device)
+    return scratch, (dev.ptr(scratch) + 255) & ~255, nbytes
+
+
 def _launch_sample_and_step(c, rg, tg, pg, pts, n: int, ds: float, ini, policy: int, out) -> None:
     """bhn_sample_and_step_stokes, or for large point sets its cell-ordered form
     (bhn_sample_and_step_stokes_sorted: the same values, neighbouring points
@@ -220,13 +279,10 @@ def _launch_sample_and_step(c, rg, tg, pg, pts, n: int, ds: float, ini, policy: 
     L = _lib.lib()
     args = (dev.ptr(c), dev.ptr(rg), rg.numel(), dev.ptr(tg), tg.numel(), dev.ptr(pg), pg.numel(), dev.ptr(pts), n, ds,
             dev.ptr(ini), ini.numel(), policy, dev.ptr(out))
-    nbytes = int(L.bhn_sample_sort_scratch_bytes(n, rg.numel() * tg.numel() * pg.numel())) if n >= SORT_MIN_POINTS \
-        else -1
-    if nbytes <= 0:
+    scratch, sp, nbytes = _sort_scratch(n, rg.numel() * tg.numel() * pg.numel(), out.device)
+    if scratch is None:
         _lib.check(L.bhn_sample_and_step_stokes(*args, dev.stream_ptr()))
         return
-    scratch = torch.empty(nbytes + 256, dtype=torch.uint8, device=out.device)
-    sp = (dev.ptr(scratch) + 255) & ~255
     _lib.check(L.bhn_sample_and_step_stokes_sorted(*args, sp, nbytes, dev.stream_ptr()))
 
 
@@ -235,13 +291,10 @@ def _launch_sample_trilinear(c, rg, tg, pg, pts, n: int, out) -> None:
     L = _lib.lib()
     args = (dev.ptr(c), dev.ptr(rg), rg.numel(), dev.ptr(tg), tg.numel(), dev.ptr(pg), pg.numel(), dev.ptr(pts), n,
             dev.ptr(out))
-    nbytes = int(L.bhn_sample_sort_scratch_bytes(n, rg.numel() * tg.numel() * pg.numel())) if n >= SORT_MIN_POINTS \
-        else -1
-    if nbytes <= 0:
+    scratch, sp, nbytes = _sort_scratch(n, rg.numel() * tg.numel() * pg.numel(), out.device)
+    if scratch is None:
         _lib.check(L.bhn_sample_brick_trilinear(*args, dev.stream_ptr()))
         return
-    scratch = torch.empty(nbytes + 256, dtype=torch.uint8, device=out.device)
-    sp = (dev.ptr(scratch) + 255) & ~255
     _lib.check(L.bhn_sample_brick_trilinear_sorted(*args, sp, nbytes, dev.stream_ptr()))
 
 

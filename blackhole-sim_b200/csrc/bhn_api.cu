@@ -8,6 +8,7 @@
 // core's (native/core/src/lib.rs) bit for bit.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <mutex>
@@ -16,6 +17,7 @@
 #include "bhn_internal.cuh"
 #include "bhn_transfer.cuh"
 #include "bhn_exact.cuh"
+#include "bhn_sampler.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
 
@@ -91,127 +93,42 @@ void stream_free(void *p, cudaStream_t s) {
 // exact helpers: bhn_exact.cuh
 
 // ------------------------------------------------------------------- kernels
-__global__ void stokes_rk2_brick_kernel(const double *__restrict__ coeffs, int64_t cells, double ds,
-                                        const double *__restrict__ initial, int broadcast, double *__restrict__ out) {
+// One Stokes step per cell (EXACT: the matrix exponential; else RK2).  counts,
+// when given: += non-finite coefficients and initial values, which saves the
+// checked call a pass over both.
+template <bool EXACT>
+__global__ void __launch_bounds__(EXACT ? 128 : 256) stokes_brick_kernel(const double *__restrict__ coeffs,
+                                                                         int64_t cells, double ds,
+                                                                         const double *__restrict__ initial,
+                                                                         int broadcast, double *__restrict__ out,
+                                                                         uint32_t *counts) {
+    uint32_t bad_c = 0, bad_s = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < cells; i += (int64_t)gridDim.x * blockDim.x) {
         double c[11];
 #pragma unroll
         for (int k = 0; k < 11; ++k) c[k] = coeffs[11 * i + k];
         const double *s0 = initial + (broadcast ? 0 : 4 * i);
         double s[4] = {s0[0], s0[1], s0[2], s0[3]};
-        stokes_step_rk2_exact(s, c, ds);
-        reinterpret_cast<double2 *>(out + 4 * i)[0] = make_double2(s[0], s[1]);
-        reinterpret_cast<double2 *>(out + 4 * i)[1] = make_double2(s[2], s[3]);
-    }
-}
-
-__global__ void stokes_exact_brick_kernel(const double *__restrict__ coeffs, int64_t cells, double ds,
-                                          const double *__restrict__ initial, int broadcast, double *__restrict__ out) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < cells; i += (int64_t)gridDim.x * blockDim.x) {
-        double c[11];
+        if (counts) {
 #pragma unroll
-        for (int k = 0; k < 11; ++k) c[k] = coeffs[11 * i + k];
-        const double *s0 = initial + (broadcast ? 0 : 4 * i);
-        double s[4] = {s0[0], s0[1], s0[2], s0[3]};
-        stokes_step_exact(s, c, ds);
-        reinterpret_cast<double2 *>(out + 4 * i)[0] = make_double2(s[0], s[1]);
-        reinterpret_cast<double2 *>(out + 4 * i)[1] = make_double2(s[2], s[3]);
-    }
-}
-
-__device__ __forceinline__ void sample_trilinear_point(const double *__restrict__ coeffs, const double *__restrict__ rg,
-                                                       int nr, const double *__restrict__ tg, int nt,
-                                                       const double *__restrict__ pg, int np,
-                                                       const double *__restrict__ pts, int64_t i,
-                                                       double *__restrict__ out) {
-    double c[11];
-    if (!sample_one_exact(coeffs, rg, nr, tg, nt, pg, np, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], c)) {
+            for (int k = 0; k < 11; ++k) bad_c += !isfinite(c[k]);
 #pragma unroll
-        for (int k = 0; k < 11; ++k) c[k] = __longlong_as_double(0x7ff8000000000000ULL);
-    }
-#pragma unroll
-    for (int k = 0; k < 11; ++k) out[11 * i + k] = c[k];
-}
-
-__global__ void sample_trilinear_kernel(const double *__restrict__ coeffs, const double *__restrict__ rg, int nr,
-                                        const double *__restrict__ tg, int nt, const double *__restrict__ pg, int np,
-                                        const double *__restrict__ pts, int64_t n, double *__restrict__ out) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        sample_trilinear_point(coeffs, rg, nr, tg, nt, pg, np, pts, i, out);
-}
-
-__global__ void sample_trilinear_ordered_kernel(const double *__restrict__ coeffs, const double *__restrict__ rg,
-                                                int nr, const double *__restrict__ tg, int nt,
-                                                const double *__restrict__ pg, int np, const double *__restrict__ pts,
-                                                const uint32_t *__restrict__ order, int64_t n,
-                                                double *__restrict__ out) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-        sample_trilinear_point(coeffs, rg, nr, tg, nt, pg, np, pts, (int64_t)order[k], out);
-}
-
-__global__ void sample_and_step_kernel(const double *__restrict__ coeffs, const double *__restrict__ rg, int nr,
-                                       const double *__restrict__ tg, int nt, const double *__restrict__ pg, int np,
-                                       const double *__restrict__ pts, int64_t n, double ds,
-                                       const double *__restrict__ initial, int broadcast, int policy,
-                                       double *__restrict__ out);
-
-// One Stokes RK2 sample-and-step of point i (native_kernels.py:325-407 with the policy of :391-397).
-__device__ __forceinline__ void sample_and_step_point(const double *__restrict__ coeffs, const double *__restrict__ rg,
-                                                      int nr, const double *__restrict__ tg, int nt,
-                                                      const double *__restrict__ pg, int np,
-                                                      const double *__restrict__ pts, int64_t i, double ds,
-                                                      const double *__restrict__ initial, int broadcast, int policy,
-                                                      double *__restrict__ out) {
-    double c[11];
-    const double *s0 = initial + (broadcast ? 0 : 4 * i);
-    double s[4] = {s0[0], s0[1], s0[2], s0[3]};
-    if (sample_one_exact(coeffs, rg, nr, tg, nt, pg, np, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], c)) {
-        stokes_step_rk2_exact(s, c, ds);
-    } else if (policy == BHN_POLICY_ZERO) {
-        s[0] = s[1] = s[2] = s[3] = 0.0;
-    } else if (policy != BHN_POLICY_INITIAL) {
-        s[0] = s[1] = s[2] = s[3] = __longlong_as_double(0x7ff8000000000000ULL);
-    }
-    reinterpret_cast<double2 *>(out + 4 * i)[0] = make_double2(s[0], s[1]);
-    reinterpret_cast<double2 *>(out + 4 * i)[1] = make_double2(s[2], s[3]);
-}
-
-// The cell (r0, theta0, phi0) a point samples from, as one index; points the
-// sampler rejects (outside the nonperiodic r/theta range, non-finite) sort last.
-__global__ void cell_key_kernel(const double *__restrict__ rg, int nr, const double *__restrict__ tg, int nt,
-                                const double *__restrict__ pg, int np, const double *__restrict__ pts, int64_t n,
-                                uint32_t invalid_key, uint32_t *__restrict__ keys, uint32_t *__restrict__ idx) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        int r0, t0, p0, p1;
-        double wr, wt, wp;
-        uint32_t key = invalid_key;
-        if (bracket_linear_exact(rg, nr, pts[3 * i], r0, wr) && bracket_linear_exact(tg, nt, pts[3 * i + 1], t0, wt)) {
-            bracket_phi_exact(pg, np, pts[3 * i + 2], p0, p1, wp);
-            key = (uint32_t)(((int64_t)r0 * nt + t0) * np + p0);
+            for (int k = 0; k < 4; ++k) bad_s += !isfinite(s[k]);
         }
-        keys[i] = key;
-        idx[i] = (uint32_t)i;
+        if constexpr (EXACT)
+            stokes_step_exact(s, c, ds);
+        else
+            stokes_step_rk2_exact(s, c, ds);
+        reinterpret_cast<double2 *>(out + 4 * i)[0] = make_double2(s[0], s[1]);
+        reinterpret_cast<double2 *>(out + 4 * i)[1] = make_double2(s[2], s[3]);
     }
-}
-
-__global__ void sample_and_step_kernel(const double *__restrict__ coeffs, const double *__restrict__ rg, int nr,
-                                       const double *__restrict__ tg, int nt, const double *__restrict__ pg, int np,
-                                       const double *__restrict__ pts, int64_t n, double ds,
-                                       const double *__restrict__ initial, int broadcast, int policy,
-                                       double *__restrict__ out) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        sample_and_step_point(coeffs, rg, nr, tg, nt, pg, np, pts, i, ds, initial, broadcast, policy, out);
-}
-
-__global__ void sample_and_step_ordered_kernel(const double *__restrict__ coeffs, const double *__restrict__ rg,
-                                               int nr, const double *__restrict__ tg, int nt,
-                                               const double *__restrict__ pg, int np, const double *__restrict__ pts,
-                                               const uint32_t *__restrict__ order, int64_t n, double ds,
-                                               const double *__restrict__ initial, int broadcast, int policy,
-                                               double *__restrict__ out) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-        sample_and_step_point(coeffs, rg, nr, tg, nt, pg, np, pts, (int64_t)order[k], ds, initial, broadcast, policy,
-                              out);
+    if (!counts) return;
+    bad_c = __reduce_add_sync(0xffffffffu, bad_c);
+    bad_s = __reduce_add_sync(0xffffffffu, bad_s);
+    if ((threadIdx.x & 31) == 0) {
+        if (bad_c) atomicAdd(counts, bad_c);
+        if (bad_s) atomicAdd(counts + 1, bad_s);
+    }
 }
 
 __global__ void valid_mask_kernel(const double *__restrict__ rg, int nr, const double *__restrict__ tg, int nt,
@@ -432,66 +349,116 @@ int bhn_device_info(int32_t *sm_count, int32_t *cc_major, int32_t *cc_minor, int
     return BHN_OK;
 }
 
-int bhn_stokes_rk2_brick(const double *coeffs, int64_t cells, double ds_cm, const double *initial, int64_t initial_len,
-                         double *out, void *stream) {
+namespace {
+int launch_stokes_brick(const double *coeffs, int64_t cells, double ds_cm, const double *initial, int64_t initial_len,
+                        bool exact, double *out, uint32_t *counts, void *stream) {
     if (!std::isfinite(ds_cm) || ds_cm < 0.0) return fail(BHN_ERR_VALUE, "ds_cm must be finite and non-negative");
     if (cells <= 0) return fail(BHN_ERR_VALUE, "coeffs must contain one or more flat 11-coefficient cells");
     if (initial_len != 4 && initial_len != 4 * cells)
         return fail(BHN_ERR_VALUE, "initial must contain either 4 values or 4 values per coefficient cell");
-    stokes_rk2_brick_kernel<<<grid_for(cells, 256), 256, 0, as_stream(stream)>>>(coeffs, cells, ds_cm, initial,
-                                                                                 initial_len == 4, out);
-    BHN_LAUNCH_CHECK("stokes_rk2_brick_kernel");
+    cudaStream_t s = as_stream(stream);
+    if (counts) BHN_CUDA_TRY(cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), s));
+    if (exact)
+        stokes_brick_kernel<true><<<grid_for(cells, 128), 128, 0, s>>>(coeffs, cells, ds_cm, initial, initial_len == 4,
+                                                                       out, counts);
+    else
+        stokes_brick_kernel<false><<<grid_for(cells, 256), 256, 0, s>>>(coeffs, cells, ds_cm, initial,
+                                                                        initial_len == 4, out, counts);
+    BHN_LAUNCH_CHECK("stokes_brick_kernel");
     return BHN_OK;
+}
+
+int check_sampler_sizes(int64_t nr, int64_t nt, int64_t np, int64_t n_points) {
+    int rc = check_grid_sizes(nr, nt, np);
+    if (rc) return rc;
+    if (n_points < 0) return fail(BHN_ERR_VALUE, "points must contain flat r, theta, phi triples");
+    return BHN_OK;
+}
+
+int check_step(double ds_cm, int64_t n_points, int64_t initial_len, int32_t policy) {
+    if (!std::isfinite(ds_cm) || ds_cm < 0.0) return fail(BHN_ERR_VALUE, "ds_cm must be finite and non-negative");
+    if (policy < 0 || policy > 2) return fail(BHN_ERR_VALUE, "invalid_policy must be 'nan', 'initial', or 'zero'");
+    if (initial_len != 4 && initial_len != 4 * n_points)
+        return fail(BHN_ERR_VALUE, "initial must contain either 4 values or 4 values per sample point");
+    return BHN_OK;
+}
+
+SamplePoints sample_points(const double *coeffs, const double *rg, int64_t nr, const double *tg, int64_t nt,
+                           const double *pg, int64_t np, const double *points, int64_t n, double *out) {
+    SamplePoints P = {};
+    P.coeffs = coeffs;
+    P.rg = rg;
+    P.tg = tg;
+    P.pg = pg;
+    P.nr = (int)nr;
+    P.nt = (int)nt;
+    P.np = (int)np;
+    P.pts = points;
+    P.n = n;
+    P.out = out;
+    return P;
+}
+
+int launch_samples(const SamplePoints &P, bool step, cudaStream_t s) {
+    const int64_t groups = (P.n + 31) / 32, resident = (int64_t)std::max(1, sm_count_current_device()) * kSampleBlocks;
+    const int threads = (int)std::min<int64_t>(kSampleThreads, 32 * std::max<int64_t>(2, (groups + resident - 1) / resident));
+    const int64_t blocks = std::min(resident, (32 * groups + threads - 1) / threads);
+    const int smem = (int)sizeof(WarpPoints) * (threads / 32) + grid_smem(P.nr, P.nt, P.np);
+    auto go = [&](auto kernel) -> int {
+        if (smem > 48 * 1024)
+            BHN_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        kernel<<<(unsigned)blocks, threads, smem, s>>>(P);
+        BHN_LAUNCH_CHECK("sample_points_kernel");
+        return BHN_OK;
+    };
+    if (step) return P.order ? go(sample_points_kernel<true, true>) : go(sample_points_kernel<true, false>);
+    return P.order ? go(sample_points_kernel<false, true>) : go(sample_points_kernel<false, false>);
+}
+}  // namespace
+
+int bhn_stokes_rk2_brick(const double *coeffs, int64_t cells, double ds_cm, const double *initial, int64_t initial_len,
+                         double *out, void *stream) {
+    return launch_stokes_brick(coeffs, cells, ds_cm, initial, initial_len, false, out, nullptr, stream);
 }
 
 int bhn_stokes_exact_brick(const double *coeffs, int64_t cells, double ds_cm, const double *initial,
                            int64_t initial_len, double *out, void *stream) {
-    if (!std::isfinite(ds_cm) || ds_cm < 0.0) return fail(BHN_ERR_VALUE, "ds_cm must be finite and non-negative");
-    if (cells <= 0) return fail(BHN_ERR_VALUE, "coeffs must contain one or more flat 11-coefficient cells");
-    if (initial_len != 4 && initial_len != 4 * cells)
-        return fail(BHN_ERR_VALUE, "initial must contain either 4 values or 4 values per coefficient cell");
-    stokes_exact_brick_kernel<<<grid_for(cells, 128), 128, 0, as_stream(stream)>>>(coeffs, cells, ds_cm, initial,
-                                                                                   initial_len == 4, out);
-    BHN_LAUNCH_CHECK("stokes_exact_brick_kernel");
-    return BHN_OK;
+    return launch_stokes_brick(coeffs, cells, ds_cm, initial, initial_len, true, out, nullptr, stream);
+}
+
+int bhn_stokes_brick_checked(const double *coeffs, int64_t cells, double ds_cm, const double *initial,
+                             int64_t initial_len, int32_t exact, double *out, uint32_t *counts, void *stream) {
+    if (!counts) return fail(BHN_ERR_VALUE, "counts must not be NULL");
+    return launch_stokes_brick(coeffs, cells, ds_cm, initial, initial_len, exact != 0, out, counts, stream);
 }
 
 int bhn_sample_brick_trilinear(const double *coeffs, const double *r_grid, int64_t nr, const double *theta_grid,
                                int64_t nt, const double *phi_grid, int64_t np, const double *points, int64_t n_points,
                                double *out, void *stream) {
-    int rc = check_grid_sizes(nr, nt, np);
-    if (rc) return rc;
-    if (n_points < 0) return fail(BHN_ERR_VALUE, "points must contain flat r, theta, phi triples");
-    if (n_points == 0) return BHN_OK;
-    sample_trilinear_kernel<<<grid_for(n_points, 128), 128, 0, as_stream(stream)>>>(
-        coeffs, r_grid, (int)nr, theta_grid, (int)nt, phi_grid, (int)np, points, n_points, out);
-    BHN_LAUNCH_CHECK("sample_trilinear_kernel");
-    return BHN_OK;
+    int rc = check_sampler_sizes(nr, nt, np, n_points);
+    if (rc || n_points == 0) return rc;
+    return launch_samples(sample_points(coeffs, r_grid, nr, theta_grid, nt, phi_grid, np, points, n_points, out), false,
+                          as_stream(stream));
 }
 
 int bhn_sample_and_step_stokes(const double *coeffs, const double *r_grid, int64_t nr, const double *theta_grid,
                                int64_t nt, const double *phi_grid, int64_t np, const double *points, int64_t n_points,
                                double ds_cm, const double *initial, int64_t initial_len, int32_t invalid_policy,
                                double *out, void *stream) {
-    if (!std::isfinite(ds_cm) || ds_cm < 0.0) return fail(BHN_ERR_VALUE, "ds_cm must be finite and non-negative");
-    int rc = check_grid_sizes(nr, nt, np);
-    if (rc) return rc;
-    if (invalid_policy < 0 || invalid_policy > 2)
-        return fail(BHN_ERR_VALUE, "invalid_policy must be 'nan', 'initial', or 'zero'");
-    if (n_points < 0) return fail(BHN_ERR_VALUE, "points must contain flat r, theta, phi triples");
-    if (initial_len != 4 && initial_len != 4 * n_points)
-        return fail(BHN_ERR_VALUE, "initial must contain either 4 values or 4 values per sample point");
-    if (n_points == 0) return BHN_OK;
-    sample_and_step_kernel<<<grid_for(n_points, 128), 128, 0, as_stream(stream)>>>(
-        coeffs, r_grid, (int)nr, theta_grid, (int)nt, phi_grid, (int)np, points, n_points, ds_cm, initial,
-        initial_len == 4, invalid_policy, out);
-    BHN_LAUNCH_CHECK("sample_and_step_kernel");
-    return BHN_OK;
+    int rc = check_sampler_sizes(nr, nt, np, n_points);
+    if (!rc) rc = check_step(ds_cm, n_points, initial_len, invalid_policy);
+    if (rc || n_points == 0) return rc;
+    SamplePoints P = sample_points(coeffs, r_grid, nr, theta_grid, nt, phi_grid, np, points, n_points, out);
+    P.initial = initial;
+    P.broadcast = initial_len == 4;
+    P.policy = invalid_policy;
+    P.ds = ds_cm;
+    return launch_samples(P, true, as_stream(stream));
 }
 
 namespace {
 struct SortLayout {
-    int64_t keys_in, keys_out, idx_in, idx_out, temp, temp_bytes, total;
+    int64_t keys_in, keys_out, idx_in, idx_out, hints, temp, temp_bytes, total;
 };
 
 int key_bits(uint32_t max_key) {
@@ -517,9 +484,10 @@ SortLayout sort_layout(int64_t n, int64_t cells) {
     L.keys_out = a;
     L.idx_in = 2 * a;
     L.idx_out = 3 * a;
-    L.temp = 4 * a;
+    L.hints = 4 * a;
+    L.temp = L.hints + up((int64_t)sizeof(AxisHints));
     L.temp_bytes = (int64_t)temp;
-    L.total = 4 * a + up((int64_t)temp);
+    L.total = L.temp + up((int64_t)temp);
     return L;
 }
 }  // namespace
@@ -527,26 +495,28 @@ SortLayout sort_layout(int64_t n, int64_t cells) {
 int64_t bhn_sample_sort_scratch_bytes(int64_t n_points, int64_t cells) { return sort_layout(n_points, cells).total; }
 
 namespace {
-// The cell keys and their radix sort: idx_out (inside the scratch) receives the
-// point indices in cell order.
-int order_points_by_cell(const double *r_grid, int64_t nr, const double *theta_grid, int64_t nt, const double *phi_grid,
-                         int64_t np, const double *points, int64_t n_points, const SortLayout &L, void *scratch,
-                         void *stream, const uint32_t *&idx_out) {
+// The cell keys and their radix sort: P.order (inside the scratch) receives the
+// point indices in cell order, P.keys the sorted keys.
+int order_points_by_cell(SamplePoints &P, const SortLayout &L, void *scratch, cudaStream_t s) {
     unsigned char *base = static_cast<unsigned char *>(scratch);
     uint32_t *keys_in = reinterpret_cast<uint32_t *>(base + L.keys_in);
     uint32_t *keys_out = reinterpret_cast<uint32_t *>(base + L.keys_out);
     uint32_t *idx_in = reinterpret_cast<uint32_t *>(base + L.idx_in);
     uint32_t *idx_sorted = reinterpret_cast<uint32_t *>(base + L.idx_out);
-    const uint32_t cells = (uint32_t)(nr * nt * np);
-    cudaStream_t s = as_stream(stream);
-    cell_key_kernel<<<grid_for(n_points, 256), 256, 0, s>>>(r_grid, (int)nr, theta_grid, (int)nt, phi_grid, (int)np,
-                                                          points, n_points, cells, keys_in, idx_in);
+    const uint32_t cells = (uint32_t)((int64_t)P.nr * P.nt * P.np);
+    AxisHints *hints = reinterpret_cast<AxisHints *>(base + L.hints);
+    axis_hints_kernel<<<1, 32, 0, s>>>(P.rg, P.nr, P.tg, P.nt, P.pg, P.np, hints);
+    BHN_LAUNCH_CHECK("axis_hints_kernel");
+    cell_key_kernel<<<grid_for(P.n, 256), 256, grid_smem(P.nr, P.nt, P.np), s>>>(
+        P.rg, P.nr, P.tg, P.nt, P.pg, P.np, P.pts, P.n, cells, hints, keys_in, idx_in, P.bad_points);
     BHN_LAUNCH_CHECK("cell_key_kernel");
     size_t temp = (size_t)L.temp_bytes;
-    if (cub::DeviceRadixSort::SortPairs(base + L.temp, temp, keys_in, keys_out, idx_in, idx_sorted, (int)n_points, 0,
+    if (cub::DeviceRadixSort::SortPairs(base + L.temp, temp, keys_in, keys_out, idx_in, idx_sorted, (int)P.n, 0,
                                         key_bits(cells), s) != cudaSuccess)
         return fail(BHN_ERR_CUDA, "radix sort of the point cells failed");
-    idx_out = idx_sorted;
+    P.keys = keys_out;
+    P.order = idx_sorted;
+    P.invalid_key = cells;
     return BHN_OK;
 }
 
@@ -563,20 +533,14 @@ int bhn_sample_brick_trilinear_sorted(const double *coeffs, const double *r_grid
                                       int64_t nt, const double *phi_grid, int64_t np, const double *points,
                                       int64_t n_points, double *out, void *scratch, int64_t scratch_bytes,
                                       void *stream) {
-    int rc = check_grid_sizes(nr, nt, np);
-    if (rc) return rc;
-    if (n_points < 0) return fail(BHN_ERR_VALUE, "points must contain flat r, theta, phi triples");
-    if (n_points == 0) return BHN_OK;
+    int rc = check_sampler_sizes(nr, nt, np, n_points);
+    if (rc || n_points == 0) return rc;
     SortLayout L;
     rc = check_sort_scratch(n_points, nr * nt * np, scratch, scratch_bytes, L);
     if (rc) return rc;
-    const uint32_t *order = nullptr;
-    rc = order_points_by_cell(r_grid, nr, theta_grid, nt, phi_grid, np, points, n_points, L, scratch, stream, order);
-    if (rc) return rc;
-    sample_trilinear_ordered_kernel<<<grid_for(n_points, 128), 128, 0, as_stream(stream)>>>(
-        coeffs, r_grid, (int)nr, theta_grid, (int)nt, phi_grid, (int)np, points, order, n_points, out);
-    BHN_LAUNCH_CHECK("sample_trilinear_ordered_kernel");
-    return BHN_OK;
+    SamplePoints P = sample_points(coeffs, r_grid, nr, theta_grid, nt, phi_grid, np, points, n_points, out);
+    rc = order_points_by_cell(P, L, scratch, as_stream(stream));
+    return rc ? rc : launch_samples(P, false, as_stream(stream));
 }
 
 int bhn_sample_and_step_stokes_sorted(const double *coeffs, const double *r_grid, int64_t nr,
@@ -584,27 +548,61 @@ int bhn_sample_and_step_stokes_sorted(const double *coeffs, const double *r_grid
                                       const double *points, int64_t n_points, double ds_cm, const double *initial,
                                       int64_t initial_len, int32_t invalid_policy, double *out, void *scratch,
                                       int64_t scratch_bytes, void *stream) {
-    if (!std::isfinite(ds_cm) || ds_cm < 0.0) return fail(BHN_ERR_VALUE, "ds_cm must be finite and non-negative");
-    int rc = check_grid_sizes(nr, nt, np);
-    if (rc) return rc;
-    if (invalid_policy < 0 || invalid_policy > 2)
-        return fail(BHN_ERR_VALUE, "invalid_policy must be 'nan', 'initial', or 'zero'");
-    if (n_points < 0) return fail(BHN_ERR_VALUE, "points must contain flat r, theta, phi triples");
-    if (initial_len != 4 && initial_len != 4 * n_points)
-        return fail(BHN_ERR_VALUE, "initial must contain either 4 values or 4 values per sample point");
-    if (n_points == 0) return BHN_OK;
+    int rc = check_sampler_sizes(nr, nt, np, n_points);
+    if (!rc) rc = check_step(ds_cm, n_points, initial_len, invalid_policy);
+    if (rc || n_points == 0) return rc;
     SortLayout L;
     rc = check_sort_scratch(n_points, nr * nt * np, scratch, scratch_bytes, L);
     if (rc) return rc;
-    const uint32_t *idx_out = nullptr;
-    rc = order_points_by_cell(r_grid, nr, theta_grid, nt, phi_grid, np, points, n_points, L, scratch, stream, idx_out);
+    SamplePoints P = sample_points(coeffs, r_grid, nr, theta_grid, nt, phi_grid, np, points, n_points, out);
+    P.initial = initial;
+    P.broadcast = initial_len == 4;
+    P.policy = invalid_policy;
+    P.ds = ds_cm;
+    rc = order_points_by_cell(P, L, scratch, as_stream(stream));
+    return rc ? rc : launch_samples(P, true, as_stream(stream));
+}
+
+int bhn_sample_points_checked(const double *coeffs, const double *r_grid, int64_t nr, const double *theta_grid,
+                              int64_t nt, const double *phi_grid, int64_t np, const double *points, int64_t n_points,
+                              double ds_cm, const double *initial, int64_t initial_len, int32_t invalid_policy,
+                              double *out, void *scratch, int64_t scratch_bytes, uint32_t *counts, void *stream) {
+    int rc = check_sampler_sizes(nr, nt, np, n_points);
+    if (!rc && initial) rc = check_step(ds_cm, n_points, initial_len, invalid_policy);
     if (rc) return rc;
+    if (!counts) return fail(BHN_ERR_VALUE, "counts must not be NULL");
+    SortLayout L;
+    if (scratch && n_points > 0) {
+        rc = check_sort_scratch(n_points, nr * nt * np, scratch, scratch_bytes, L);
+        if (rc) return rc;
+    }
     cudaStream_t s = as_stream(stream);
-    sample_and_step_ordered_kernel<<<grid_for(n_points, 128), 128, 0, s>>>(
-        coeffs, r_grid, (int)nr, theta_grid, (int)nt, phi_grid, (int)np, points, idx_out, n_points, ds_cm, initial,
-        initial_len == 4, invalid_policy, out);
-    BHN_LAUNCH_CHECK("sample_and_step_ordered_kernel");
-    return BHN_OK;
+    BHN_CUDA_TRY(cudaMemsetAsync(counts, 0, 11 * sizeof(uint32_t), s));
+    CheckArrays C = {};
+    const double *v[kCheckArrays] = {r_grid, theta_grid, phi_grid, coeffs, initial};
+    const int64_t n[kCheckArrays] = {nr, nt, np, nr * nt * np * 11, initial ? initial_len : 0};
+    for (int a = 0; a < kCheckArrays; ++a) {
+        C.v[a] = v[a];
+        C.n[a] = n[a];
+        C.increasing[a] = a < 3;
+        C.first[a + 1] = C.first[a] + (n[a] + kCheckTile - 1) / kCheckTile;
+    }
+    C.counts = counts;
+    if (C.first[kCheckArrays] > INT32_MAX) return fail(BHN_ERR_VALUE, "coefficient brick shape is too large");
+    check_arrays_kernel<<<(unsigned)C.first[kCheckArrays], 256, 0, s>>>(C);
+    BHN_LAUNCH_CHECK("check_arrays_kernel");
+    if (n_points == 0) return BHN_OK;
+    SamplePoints P = sample_points(coeffs, r_grid, nr, theta_grid, nt, phi_grid, np, points, n_points, out);
+    P.initial = initial;
+    P.broadcast = initial_len == 4;
+    P.policy = invalid_policy;
+    P.ds = ds_cm;
+    P.bad_points = counts + 10;
+    if (scratch) {
+        rc = order_points_by_cell(P, L, scratch, s);
+        if (rc) return rc;
+    }
+    return launch_samples(P, initial != nullptr, s);
 }
 
 int bhn_sample_brick_valid_mask(const double *r_grid, int64_t nr, const double *theta_grid, int64_t nt,

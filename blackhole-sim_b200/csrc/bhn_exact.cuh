@@ -31,39 +31,6 @@ __device__ __forceinline__ void stokes_step_rk2_exact(double s[4], const double 
     for (int i = 0; i < 4; ++i) s[i] = add(s[i], mul(ds, k2[i]));
 }
 
-// lib.rs:75-87 / native_kernels.py:137-146
-__device__ __forceinline__ bool bracket_linear_exact(const double *g, int n, double x, int &i0, double &w) {
-    if (x < g[0] || x > g[n - 1]) return false;
-    if (x == g[n - 1]) {
-        i0 = n - 2;
-        w = 1.0;
-        return true;
-    }
-    int lo = search_right(g, 0, n, x) - 1;
-    lo = max(0, min(lo, n - 2));
-    double den = sub(g[lo + 1], g[lo]);
-    if (den < 1.0e-300) den = 1.0e-300;
-    i0 = lo;
-    w = sub(x, g[lo]) / den;
-    return true;
-}
-
-// lib.rs:93-106 / native_kernels.py:149-161
-__device__ __forceinline__ void bracket_phi_exact(const double *g, int n, double phi, int &i0, int &i1, double &w) {
-    double p = wrap_phi(phi, g[0]);
-    int lo = search_right(g, 0, n, p) - 1;
-    if (lo < 0) lo = n - 1;
-    if (lo >= n) lo = n - 1;
-    int hi_i = (lo + 1) % n;
-    double hi = hi_i > lo ? g[hi_i] : add(g[0], kTwoPi);
-    double pp = p >= g[lo] ? p : add(p, kTwoPi);
-    double den = sub(hi, g[lo]);
-    if (den < 1.0e-300) den = 1.0e-300;
-    i0 = lo;
-    i1 = hi_i;
-    w = sub(pp, g[lo]) / den;
-}
-
 // The trilinear blend of native_kernels.py:180-186: phi lerps, then theta, then r.
 __device__ __forceinline__ bool lerp_cells(const double *__restrict__ coeffs, int nt, int np, int r0, int t0, int p0,
                                            int p1, double wr, double wt, double wp, double out[11]) {
@@ -217,7 +184,7 @@ __device__ __forceinline__ int locate_phi_sel(const double *g, int n, double p, 
     return i;
 }
 
-// bracket_linear_exact with the cell found from the axis hint: the same cell
+// lib.rs:75-87 / native_kernels.py:137-146 with the cell found from the axis hint: the same cell
 // (searchsorted(side="right") - 1) and the same weight for any sorted grid.
 __device__ __forceinline__ bool bracket_linear_hinted(const double *g, int n, double x, int kind, double off,
                                                       double inv, double g0, double gn, int &i0, double &w) {
@@ -243,7 +210,7 @@ __device__ __forceinline__ bool bracket_linear_hinted(const double *g, int n, do
     return true;
 }
 
-// bracket_phi_exact with the hinted cell search.
+// lib.rs:93-106 / native_kernels.py:149-161 with the hinted cell search.
 __device__ __forceinline__ void bracket_phi_hinted(const double *g, int n, double phi, int kind, double off,
                                                    double inv, double g0, int &i0, int &i1, double &w) {
     double p = wrap_phi(phi, g0);
@@ -265,18 +232,7 @@ __device__ __forceinline__ void bracket_phi_hinted(const double *g, int n, doubl
     w = sub(pp, gl) / den;
 }
 
-// lib.rs:171-208 / native_kernels.py:164-186
-__device__ __forceinline__ bool sample_one_exact(const double *__restrict__ coeffs, const double *rg, int nr,
-                                                 const double *tg, int nt, const double *pg, int np, double r,
-                                                 double th, double ph, double out[11]) {
-    int r0, t0, p0, p1;
-    double wr, wt, wp;
-    if (!bracket_linear_exact(rg, nr, r, r0, wr) || !bracket_linear_exact(tg, nt, th, t0, wt)) return false;
-    bracket_phi_exact(pg, np, ph, p0, p1, wp);
-    return lerp_cells(coeffs, nt, np, r0, t0, p0, p1, wr, wt, wp, out);
-}
-
-// sample_one_exact with the hinted brackets (same cells, weights and values).
+// lib.rs:171-208 / native_kernels.py:164-186 with the hinted brackets (the exact search's cells, weights and values).
 __device__ __forceinline__ bool sample_one_hinted(const double *__restrict__ coeffs, const double *rg, int nr,
                                                   const double *tg, int nt, const double *pg, int np,
                                                   const AxisHints &h, double r, double th, double ph, double out[11]) {

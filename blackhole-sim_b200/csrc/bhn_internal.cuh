@@ -168,7 +168,10 @@ __device__ __forceinline__ int locate_phi_f(const float *g, int n, float p, int 
 
 // native_kernels.py:133-134 / lib.rs:89-91: ((phi - base) mod 2 pi) + base.
 __device__ __forceinline__ double wrap_phi(double phi, double base) {
-    double m = fmod(phi - base, kTwoPi);
+    // within two turns the remainder is exact without fmod: |x| < 2 pi is its own, and
+    // x -+ 2 pi of 2 pi <= |x| <= 4 pi is exact (Sterbenz)
+    double m = phi - base;
+    if (fabs(m) >= kTwoPi) m = fabs(m) < 2.0 * kTwoPi ? (m < 0.0 ? m + kTwoPi : m - kTwoPi) : fmod(m, kTwoPi);
     if (m < 0.0) m += kTwoPi;
     return m + base;
 }

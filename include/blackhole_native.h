@@ -90,6 +90,13 @@ int bhn_stokes_rk2_brick(const double *coeffs, int64_t cells, double ds_cm, cons
 int bhn_stokes_exact_brick(const double *coeffs, int64_t cells, double ds_cm, const double *initial,
                            int64_t initial_len, double *out, void *stream);
 
+/* Either step (exact != 0: the exponential) with the input checks of
+ * native/core/src/lib.rs:227-260 in the same pass: counts[0] and counts[1]
+ * receive the non-finite values among coeffs and initial.  counts: 2 device
+ * uint32.  Where either is not 0, out is not meaningful. */
+int bhn_stokes_brick_checked(const double *coeffs, int64_t cells, double ds_cm, const double *initial,
+                             int64_t initial_len, int32_t exact, double *out, uint32_t *counts, void *stream);
+
 /* Replaces sample_brick_trilinear (native/core/src/lib.rs:281-306).  coeffs:
  * nr*nt*np*11 in [r][theta][phi][11] order, points: n*3 (r, theta, phi),
  * out: n*11 with NaN rows outside the nonperiodic r/theta domain. */
@@ -124,6 +131,18 @@ int bhn_sample_and_step_stokes_sorted(const double *coeffs, const double *r_grid
                                       const double *points, int64_t n_points, double ds_cm, const double *initial,
                                       int64_t initial_len, int32_t invalid_policy, double *out, void *scratch,
                                       int64_t scratch_bytes, void *stream);
+
+/* Either sampler (initial NULL: bhn_sample_brick_trilinear; else
+ * bhn_sample_and_step_stokes), in cell order when scratch is given, with the
+ * input checks of native/core/src/lib.rs:112-169 queued before it: counts[2 a]
+ * and counts[2 a + 1] receive the non-finite values and the non-increasing
+ * neighbours of array a (r grid, theta grid, phi grid, coeffs, initial),
+ * counts[10] the points with a non-finite coordinate.  counts: 11 device
+ * uint32.  Where any is not 0, out is not meaningful. */
+int bhn_sample_points_checked(const double *coeffs, const double *r_grid, int64_t nr, const double *theta_grid,
+                              int64_t nt, const double *phi_grid, int64_t np, const double *points, int64_t n_points,
+                              double ds_cm, const double *initial, int64_t initial_len, int32_t invalid_policy,
+                              double *out, void *scratch, int64_t scratch_bytes, uint32_t *counts, void *stream);
 
 /* Replaces sample_brick_valid_mask (native_kernels.py:189-210, Python-only in
  * the reference): inclusive r/theta bounds, phi ignored.  mask: n bytes (0/1). */
