@@ -128,6 +128,7 @@ def _declare() -> ctypes.CDLL:
         "bhn_mlp_pack": ([vp, vp, vp, vp], ctypes.c_int),
         "bhn_mlp_grad": ([vp, vp, vp, i64, i64, vp, vp, vp], ctypes.c_int),
         "bhn_mlp_adam": ([vp, vp, vp, vp, f, f, f, f, i32, vp], ctypes.c_int),
+        "bhn_mlp_epoch": ([vp, vp, vp, i64, i64, vp, vp, vp, vp, ctypes.c_double, f, f, f, i64, i64, vp], ctypes.c_int),
         "bhn_mlp_infer": ([vp, vp, i64, vp, vp], ctypes.c_int),
         "bhn_adaptive_launch": ([vp, vp, i32, i32, i32, i32, cfgp, vp, rayp, vp, i64, ctypes.POINTER(AdaptStruct), vp,
                                  vp, ctypes.c_ulonglong, vp, vp], ctypes.c_int),
@@ -351,13 +352,10 @@ def train(samples: torch.Tensor, *, epochs: int = 6, batch: int = 4096, lr: floa
     for ep in range(epochs):
         index = torch.randperm(n, generator=gen, device=device)
         loss.zero_()
-        for k in range(steps_per_epoch):
-            step += 1
-            lr_t = lr * 0.5 * (1.0 + math.cos(math.pi * (step - 1) / total_steps))  # cosine decay
-            _lib.check(L.bhn_mlp_grad(dev.ptr(net.params), dev.ptr(data), dev.ptr(index), k * batch, batch,
-                                      dev.ptr(grad), dev.ptr(loss), s))
-            _lib.check(L.bhn_mlp_adam(dev.ptr(net.params), dev.ptr(grad), dev.ptr(m), dev.ptr(v), lr_t, 0.9, 0.999,
-                                      1e-8, step, s))
+        _lib.check(L.bhn_mlp_epoch(dev.ptr(net.params), dev.ptr(data), dev.ptr(index), steps_per_epoch, batch,
+                                   dev.ptr(grad), dev.ptr(loss), dev.ptr(m), dev.ptr(v), lr, 0.9, 0.999, 1e-8, step,
+                                   total_steps, s))
+        step += steps_per_epoch
         ep_loss = float(loss.item()) / (steps_per_epoch * batch)
         losses.append(ep_loss)
         if log:

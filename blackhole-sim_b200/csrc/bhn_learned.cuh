@@ -184,119 +184,174 @@ __global__ void mlp_pack_kernel(const float *__restrict__ P, MlpNorm norm, MlpBl
 }
 
 // ------------------------------------------------------------ training
-// One block = 128 samples.  Shared: BF16-rounded weights and biases, then the
-// per-sample rows x, a1, a2, dz1, dz2, dy used by the block's weight-gradient
-// reductions.  grad (FP32, kMlpParams) and loss are accumulated atomically.
-constexpr int kTrainBlock = 128;
+// One block = 32 samples, 256 threads, everything in shared memory: the
+// BF16-rounded weights and the samples' rows x, a1, a2, dz1, dz2.  The three
+// 64-wide products (forward, backward through W2, dW2) are register tiles of 2
+// x 4 or 4 x 4 outputs fed by 128-bit shared loads; rows are padded to 68
+// floats, so that both a row's and a column's neighbours lie on distinct banks.
+// Sums over a layer's inputs run in index order from the bias, as the
+// inference path's.  grad (FP32, kMlpParams) and loss are accumulated with
+// (vector) reductions.  A step of 4,096 samples fills 128 of the 148 SMs and
+// is bound by its chain of stages: 14.5 us, against 185 with a thread per sample
+// (32 blocks, every shared access a 32-way bank conflict).
+constexpr int kTrainBlock = 32, kTrainThreads = 256, kTrainRow = 68;
 constexpr int kSampleStride = 9;  // 8 standardised features + standardised target
 
-__host__ __device__ inline int64_t train_smem_bytes() {
-    return 4 * ((int64_t)kMlpParams + 3 + (int64_t)kTrainBlock * (8 + 64 * 4 + 1));
+struct __align__(16) TrainSmem {
+    float w1[8 * 64], b1[64], b2[64], w3[64], b3;
+    float dy[kTrainBlock], x[kTrainBlock][9];
+    __align__(16) float w2[64][kTrainRow];
+    float a1[kTrainBlock][kTrainRow], a2[kTrainBlock][kTrainRow];    // activations
+    float dz1[kTrainBlock][kTrainRow], dz2[kTrainBlock][kTrainRow];  // SiLU'(z), then dL/dz
+};
+
+__device__ __forceinline__ void add4(float *p, float4 v, bool vec) {
+    if (vec)
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                     : "memory");
+    else {
+        atomicAdd(p, v.x);
+        atomicAdd(p + 1, v.y);
+        atomicAdd(p + 2, v.z);
+        atomicAdd(p + 3, v.w);
+    }
+}
+__device__ __forceinline__ float4 fma4(float a, float4 b, float4 c) {
+    return make_float4(fmaf(a, b.x, c.x), fmaf(a, b.y, c.y), fmaf(a, b.z, c.z), fmaf(a, b.w, c.w));
 }
 
-__global__ void __launch_bounds__(kTrainBlock) mlp_grad_kernel(const float *__restrict__ P,
-                                                                const float *__restrict__ samples,
-                                                                const int64_t *__restrict__ index, int64_t first,
-                                                                int64_t count, float *__restrict__ grad,
-                                                                float *__restrict__ loss) {
-    extern __shared__ __align__(16) float sm[];
-    float *w = sm;                                   // kMlpParams (+3 pad)
-    float *xs = w + kMlpParams + 3;                  // [128][8]
-    float *a1s = xs + kTrainBlock * 8;               // [128][64]
-    float *a2s = a1s + kTrainBlock * 64;             // [128][64]
-    float *dz1s = a2s + kTrainBlock * 64;            // [128][64]
-    float *dz2s = dz1s + kTrainBlock * 64;           // [128][64]
-    float *dys = dz2s + kTrainBlock * 64;            // [128]
+// vec: grad is 16-byte aligned.
+__global__ void __launch_bounds__(kTrainThreads) mlp_grad_kernel(const float *__restrict__ P,
+                                                                 const float *__restrict__ samples,
+                                                                 const int64_t *__restrict__ index, int64_t first,
+                                                                 int64_t count, float *__restrict__ grad,
+                                                                 float *__restrict__ loss, bool vec) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TrainSmem &T = *reinterpret_cast<TrainSmem *>(smem_raw);
     const int tid = threadIdx.x;
-    for (int i = tid; i < kMlpParams; i += blockDim.x) {
-        const bool bias = (i >= kOffB1 && i < kOffW2) || (i >= kOffB2 && i < kOffW3) || i == kOffB3;
-        w[i] = bias ? P[i] : bf16_round(P[i]);
+    const int64_t base = (int64_t)blockIdx.x * kTrainBlock;
+    for (int e = tid; e < kTrainBlock * 9; e += kTrainThreads) {  // the samples' rows
+        const int s = e / 9, k = e - 9 * s;
+        const float v = base + s < count ? samples[index[first + base + s] * kSampleStride + k] : 0.0f;
+        T.x[s][k] = k < 8 ? bf16_round(v) : v;
     }
-    __syncthreads();
-    const int64_t s = (int64_t)blockIdx.x * kTrainBlock + tid;
-    const bool live = s < count;
-    const float *row = samples + (live ? index[first + s] : 0) * kSampleStride;
-    float x[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        x[k] = live ? bf16_round(row[k]) : 0.0f;
-        xs[tid * 8 + k] = x[k];
-    }
-    const float target = live ? row[8] : 0.0f;
-    // forward, layer 1 (z1 kept as sigmoid' in dz1s until the backward pass)
-    for (int j = 0; j < 64; j += 2) {
-        float z0 = w[kOffB1 + j], z1 = w[kOffB1 + j + 1];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            z0 = fmaf(x[k], w[kOffW1 + k * 64 + j], z0);
-            z1 = fmaf(x[k], w[kOffW1 + k * 64 + j + 1], z1);
-        }
-        float a0, a1, s0, s1;
-        silu2(z0, z1, a0, a1, s0, s1);
-        a1s[tid * 64 + j] = bf16_round(a0);
-        a1s[tid * 64 + j + 1] = bf16_round(a1);
-        dz1s[tid * 64 + j] = fmaf(z0 * s0, 1.0f - s0, s0);  // SiLU'(z) = s + z s (1 - s)
-        dz1s[tid * 64 + j + 1] = fmaf(z1 * s1, 1.0f - s1, s1);
-    }
-    // layer 2
-    float y = w[kOffB3];
-    for (int j = 0; j < 64; j += 2) {
-        float z0 = w[kOffB2 + j], z1 = w[kOffB2 + j + 1];
-        for (int i = 0; i < 64; ++i) {
-            const float a = a1s[tid * 64 + i];
-            z0 = fmaf(a, w[kOffW2 + i * 64 + j], z0);
-            z1 = fmaf(a, w[kOffW2 + i * 64 + j + 1], z1);
-        }
-        float a0, a1, s0, s1;
-        silu2(z0, z1, a0, a1, s0, s1);
-        a0 = bf16_round(a0);
-        a1 = bf16_round(a1);
-        a2s[tid * 64 + j] = a0;
-        a2s[tid * 64 + j + 1] = a1;
-        dz2s[tid * 64 + j] = fmaf(z0 * s0, 1.0f - s0, s0);
-        dz2s[tid * 64 + j + 1] = fmaf(z1 * s1, 1.0f - s1, s1);
-        y = fmaf(a0, w[kOffW3 + j], y);
-        y = fmaf(a1, w[kOffW3 + j + 1], y);
-    }
-    // backward: loss = mean (y - t)^2 over the batch
-    const float err = live ? y - target : 0.0f;
-    const float dy = 2.0f * err / (float)count;
-    dys[tid] = dy;
-    if (live) atomicAdd(loss, err * err);
-    for (int j = 0; j < 64; ++j) dz2s[tid * 64 + j] *= dy * w[kOffW3 + j];
-    for (int i = 0; i < 64; ++i) {
-        float da = 0.0f;
-        for (int j = 0; j < 64; ++j) da = fmaf(w[kOffW2 + i * 64 + j], dz2s[tid * 64 + j], da);
-        dz1s[tid * 64 + i] *= da;
-    }
-    __syncthreads();
-    // block reductions over the 128 samples
-    for (int e = tid; e < 64 * 64; e += blockDim.x) {  // dW2
-        const int i = e / 64, j = e % 64;
-        float acc = 0.0f;
-        for (int q = 0; q < kTrainBlock; ++q) acc = fmaf(a1s[q * 64 + i], dz2s[q * 64 + j], acc);
-        atomicAdd(&grad[kOffW2 + e], acc);
-    }
-    for (int e = tid; e < 8 * 64; e += blockDim.x) {  // dW1
-        const int k = e / 64, i = e % 64;
-        float acc = 0.0f;
-        for (int q = 0; q < kTrainBlock; ++q) acc = fmaf(xs[q * 8 + k], dz1s[q * 64 + i], acc);
-        atomicAdd(&grad[kOffW1 + e], acc);
-    }
+    for (int e = tid; e < 64 * 64; e += kTrainThreads) T.w2[e >> 6][e & 63] = bf16_round(P[kOffW2 + e]);
+    for (int e = tid; e < 512; e += kTrainThreads) T.w1[e] = bf16_round(P[kOffW1 + e]);
     if (tid < 64) {
-        float g1 = 0.0f, g2 = 0.0f, g3 = 0.0f;
-        for (int q = 0; q < kTrainBlock; ++q) {
-            g1 += dz1s[q * 64 + tid];
-            g2 += dz2s[q * 64 + tid];
-            g3 = fmaf(a2s[q * 64 + tid], dys[q], g3);
-        }
-        atomicAdd(&grad[kOffB1 + tid], g1);
-        atomicAdd(&grad[kOffB2 + tid], g2);
-        atomicAdd(&grad[kOffW3 + tid], g3);
+        T.b1[tid] = P[kOffB1 + tid];
+        T.b2[tid] = P[kOffB2 + tid];
+        T.w3[tid] = bf16_round(P[kOffW3 + tid]);
     }
-    if (tid == 64) {
+    if (tid == 0) T.b3 = P[kOffB3];
+    __syncthreads();
+    const int tx = tid & 15, ty = tid >> 4;
+    auto activate = [&](const float4 &z, float *a, float *ds) {  // SiLU and its derivative s + z s (1 - s)
+        const float zz[4] = {z.x, z.y, z.z, z.w};
+        float av[4], sv[4];
+        silu2(zz[0], zz[1], av[0], av[1], sv[0], sv[1]);
+        silu2(zz[2], zz[3], av[2], av[3], sv[2], sv[3]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            av[q] = bf16_round(av[q]);
+            sv[q] = fmaf(zz[q] * sv[q], 1.0f - sv[q], sv[q]);
+        }
+        *reinterpret_cast<float4 *>(a) = make_float4(av[0], av[1], av[2], av[3]);
+        *reinterpret_cast<float4 *>(ds) = make_float4(sv[0], sv[1], sv[2], sv[3]);
+    };
+    // forward, layers 1 and 2: samples 2 ty, 2 ty + 1, outputs 4 tx .. 4 tx + 3
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int s = 2 * ty + q;
+        float4 z = *reinterpret_cast<const float4 *>(&T.b1[4 * tx]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) z = fma4(T.x[s][k], *reinterpret_cast<const float4 *>(&T.w1[64 * k + 4 * tx]), z);
+        activate(z, &T.a1[s][4 * tx], &T.dz1[s][4 * tx]);
+    }
+    __syncthreads();
+    {
+        float4 z0 = *reinterpret_cast<const float4 *>(&T.b2[4 * tx]), z1 = z0;
+#pragma unroll 4
+        for (int k = 0; k < 64; k += 4) {
+            const float4 u = *reinterpret_cast<const float4 *>(&T.a1[2 * ty][k]);
+            const float4 v = *reinterpret_cast<const float4 *>(&T.a1[2 * ty + 1][k]);
+            const float uu[4] = {u.x, u.y, u.z, u.w}, vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 w = *reinterpret_cast<const float4 *>(&T.w2[k + q][4 * tx]);
+                z0 = fma4(uu[q], w, z0);
+                z1 = fma4(vv[q], w, z1);
+            }
+        }
+        activate(z0, &T.a2[2 * ty][4 * tx], &T.dz2[2 * ty][4 * tx]);
+        activate(z1, &T.a2[2 * ty + 1][4 * tx], &T.dz2[2 * ty + 1][4 * tx]);
+    }
+    __syncthreads();
+    // the output and loss = mean (y - t)^2 over the batch
+    if (tid < kTrainBlock) {
+        float y = T.b3;
+        for (int j = 0; j < 64; ++j) y = fmaf(T.a2[tid][j], T.w3[j], y);
+        const bool live = base + tid < count;
+        const float err = live ? y - T.x[tid][8] : 0.0f;
+        T.dy[tid] = 2.0f * err / (float)count;
+        // one addition per sample: the epoch's float sum loses the same small terms however the samples are blocked
+        // (partial sums moved the reported loss by up to 1.5e-4 at 200,000 samples)
+        if (live) atomicAdd(loss, err * err);
+    }
+    __syncthreads();
+    for (int e = tid; e < kTrainBlock * 64; e += kTrainThreads) {
+        const int s = e >> 6, j = e & 63;
+        T.dz2[s][j] *= T.dy[s] * T.w3[j];
+    }
+    __syncthreads();
+    {   // back through W2: inputs tx + 16 m of samples 2 ty, 2 ty + 1
+        float d[2][4] = {};
+#pragma unroll 4
+        for (int j = 0; j < 64; j += 4) {
+            const float4 u = *reinterpret_cast<const float4 *>(&T.dz2[2 * ty][j]);
+            const float4 v = *reinterpret_cast<const float4 *>(&T.dz2[2 * ty + 1][j]);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const float4 w = *reinterpret_cast<const float4 *>(&T.w2[tx + 16 * m][j]);
+                d[0][m] = fmaf(w.w, u.w, fmaf(w.z, u.z, fmaf(w.y, u.y, fmaf(w.x, u.x, d[0][m]))));
+                d[1][m] = fmaf(w.w, v.w, fmaf(w.z, v.z, fmaf(w.y, v.y, fmaf(w.x, v.x, d[1][m]))));
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int m = 0; m < 4; ++m) T.dz1[2 * ty + q][tx + 16 * m] *= d[q][m];
+    }
+    __syncthreads();
+    {   // dW2: rows 4 ty .. 4 ty + 3, columns 4 tx .. 4 tx + 3
+        float4 g[4] = {};
+#pragma unroll 4
+        for (int s = 0; s < kTrainBlock; ++s) {
+            const float4 a = *reinterpret_cast<const float4 *>(&T.a1[s][4 * ty]);
+            const float4 d = *reinterpret_cast<const float4 *>(&T.dz2[s][4 * tx]);
+            g[0] = fma4(a.x, d, g[0]);
+            g[1] = fma4(a.y, d, g[1]);
+            g[2] = fma4(a.z, d, g[2]);
+            g[3] = fma4(a.w, d, g[3]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) add4(&grad[kOffW2 + 64 * (4 * ty + q) + 4 * tx], g[q], vec);
+    }
+    if (tid < 128) {  // dW1: input tid / 16, columns 4 tx
+        float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int s = 0; s < kTrainBlock; ++s)
+            g = fma4(T.x[s][ty], *reinterpret_cast<const float4 *>(&T.dz1[s][4 * tx]), g);
+        add4(&grad[kOffW1 + 64 * ty + 4 * tx], g, vec);
+    } else if (tid < 176) {  // db1, db2, dW3
+        const int which = ty - 8;
+        float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int s = 0; s < kTrainBlock; ++s) {
+            const float *row = which == 0 ? T.dz1[s] : (which == 1 ? T.dz2[s] : T.a2[s]);
+            g = fma4(which == 2 ? T.dy[s] : 1.0f, *reinterpret_cast<const float4 *>(&row[4 * tx]), g);
+        }
+        add4(&grad[(which == 0 ? kOffB1 : (which == 1 ? kOffB2 : kOffW3)) + 4 * tx], g, vec);
+    } else if (tid == 176) {  // db3
         float g = 0.0f;
-        for (int q = 0; q < kTrainBlock; ++q) g += dys[q];
+        for (int s = 0; s < kTrainBlock; ++s) g += T.dy[s];
         atomicAdd(&grad[kOffB3], g);
     }
 }
@@ -1008,10 +1063,11 @@ int bhn_mlp_pack(const float *params, const float *h_norm, void *blob, void *str
 int bhn_mlp_grad(const float *params, const float *samples, const int64_t *index, int64_t first, int64_t count,
                  float *grad, float *loss, void *stream) {
     if (count < 1) return fail(BHN_ERR_VALUE, "batch must contain at least one sample");
-    const int smem = (int)train_smem_bytes();
+    const int smem = (int)sizeof(TrainSmem);
     BHN_CUDA_TRY(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     const unsigned blocks = (unsigned)((count + kTrainBlock - 1) / kTrainBlock);
-    mlp_grad_kernel<<<blocks, kTrainBlock, smem, as_stream(stream)>>>(params, samples, index, first, count, grad, loss);
+    mlp_grad_kernel<<<blocks, kTrainThreads, smem, as_stream(stream)>>>(
+        params, samples, index, first, count, grad, loss, (reinterpret_cast<uintptr_t>(grad) & 15) == 0);
     BHN_LAUNCH_CHECK("mlp_grad_kernel");
     return BHN_OK;
 }
@@ -1023,6 +1079,21 @@ int bhn_mlp_adam(float *params, float *grad, float *m, float *v, float lr, float
     mlp_adam_kernel<<<(kMlpParams + 255) / 256, 256, 0, as_stream(stream)>>>(params, grad, m, v, lr, beta1, beta2,
                                                                              eps, bc1, bc2);
     BHN_LAUNCH_CHECK("mlp_adam_kernel");
+    return BHN_OK;
+}
+
+int bhn_mlp_epoch(float *params, const float *samples, const int64_t *index, int64_t steps, int64_t batch, float *grad,
+                  float *loss, float *m, float *v, double lr, float beta1, float beta2, float eps, int64_t step,
+                  int64_t total_steps, void *stream) {
+    if (steps < 0 || step < 0 || total_steps < step + steps || step + steps > INT32_MAX)
+        return fail(BHN_ERR_VALUE, "an epoch needs 0 <= steps and step + steps <= total_steps");
+    for (int64_t k = 0; k < steps; ++k) {
+        int rc = bhn_mlp_grad(params, samples, index, k * batch, batch, grad, loss, stream);
+        if (rc) return rc;
+        const double lr_t = lr * 0.5 * (1.0 + cos(kPi * (double)(step + k) / (double)total_steps));  // cosine decay
+        rc = bhn_mlp_adam(params, grad, m, v, (float)lr_t, beta1, beta2, eps, (int32_t)(step + k + 1), stream);
+        if (rc) return rc;
+    }
     return BHN_OK;
 }
 

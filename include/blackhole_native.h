@@ -336,6 +336,12 @@ int bhn_mlp_grad(const float *params, const float *samples, const int64_t *index
 /* One Adam step (step counts from 1); clears grad. */
 int bhn_mlp_adam(float *params, float *grad, float *m, float *v, float lr, float beta1, float beta2, float eps,
                  int32_t step, void *stream);
+/* Steps step + 1 .. step + steps of a training run in one call: step k takes
+ * index[k batch .. (k + 1) batch) through bhn_mlp_grad and bhn_mlp_adam with the
+ * rate lr (1 + cos(pi (step + k) / total_steps)) / 2. */
+int bhn_mlp_epoch(float *params, const float *samples, const int64_t *index, int64_t steps, int64_t batch, float *grad,
+                  float *loss, float *m, float *v, double lr, float beta1, float beta2, float eps, int64_t step,
+                  int64_t total_steps, void *stream);
 /* The inference path on given standardised feature rows (n x 8) -> n outputs. */
 int bhn_mlp_infer(const void *blob, const float *features, int64_t n, float *out, void *stream);
 /* Step-doubling controller over prepared views (bhn_render_prepare): float4
