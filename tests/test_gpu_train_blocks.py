@@ -24,7 +24,7 @@ def _setup(n, seed=0):
     norm[8:16] = norm[17] = 1.0
     net = learned.StepNet.initial(norm, seed=seed)
     rows = torch.from_numpy(np.random.default_rng(seed).normal(size=(n, 9)).astype(np.float32)).cuda()
-    return net, rows, torch.randperm(n, device="cuda")
+    return net, rows, torch.from_numpy(np.random.default_rng(seed + 1).permutation(n)).cuda()
 
 
 def _grad(net, rows, index, first, count, shift=0):
