@@ -344,6 +344,9 @@ def train(samples: torch.Tensor, *, epochs: int = 6, batch: int = 4096, lr: floa
     gen = torch.Generator(device=device)
     gen.manual_seed(seed)
     n = data.shape[0]
+    if n < 1 and epochs > 0:
+        raise ValueError("training needs at least one sample")
+    batch = min(batch, max(n, 1))  # a batch larger than the samples would read past the index's end
     steps_per_epoch = max(1, n // batch)
     total_steps = epochs * steps_per_epoch
     step = 0

@@ -81,3 +81,12 @@ def test_epoch_call_takes_the_single_steps():
     net, rows, index = _setup(300)
     assert L.bhn_mlp_epoch(dev.ptr(net.params), dev.ptr(rows), dev.ptr(index), 3, 100, None, None, None, None, 1e-3, 0.9,
                            0.999, 1e-8, 7, 9, dev.stream_ptr()) == 1
+
+
+def test_fewer_samples_than_a_batch():
+    """A batch is never larger than the samples: the same steps as with the batch given as their number."""
+    rows = torch.from_numpy(np.random.default_rng(2).normal(size=(70, 9)).astype(np.float32)).cuda()
+    a, b = (learned.train(rows, epochs=2, batch=n, seed=1) for n in (4096, 70))
+    assert np.allclose(a.losses, b.losses, rtol=1e-4) and len(a.losses) == 2
+    with pytest.raises(ValueError, match="at least one sample"):
+        learned.train(rows[:0], epochs=1)
