@@ -699,7 +699,7 @@ __device__ __forceinline__ void stage_shared(const RenderParams &P, unsigned cha
         c.esc = (float)v.escape_radius;
         c.r_guard = (float)fmin(v.r_photon, T.gr[0]);  // the adaptive and learned tracers always guard the horizon
         c.r_near = 0.0f;
-        c.pad = 0.0f;
+        c.r_far = 0.0f;
         c.max_steps = v.max_steps;
         c.pad1 = c.pad2 = c.pad3 = 0;
         sconst[i] = c;

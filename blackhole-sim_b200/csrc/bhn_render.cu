@@ -225,7 +225,8 @@ struct __align__(16) StepConst {
     float a, a2, dpm, hs;               // spin, spin^2, r+ - r-, step scale
     float hmin, hmax, L, max_tau;
     float rp_h, rp_l, rcap_h, rcap_l;   // r+ and the capture radius as float pairs (value = hi + lo)
-    float esc, r_guard, r_near, pad;    // escape radius, horizon-guard radius (0 = off), FP64-island radius
+    float esc, r_guard, r_near, r_far;  // escape radius, horizon-guard radius (0 = off), FP64-island radius,
+                                        // and the radius beyond which no step's rule but escape can apply
     int max_steps, pad1, pad2, pad3;
 };
 
@@ -320,6 +321,8 @@ constexpr float kPoleIsland = 1.0e-4f;
 constexpr float kMomentumIsland = 1.0e15f;
 // Tracer32::step's answer for a step that belongs to an FP64 island.
 constexpr int kNeedFp64 = -2;
+// Its answer for a ray that has passed Tracer32::leave moving out.
+constexpr int kLeft = -3;
 
 // ------------------------------------------------------------ FP64 helpers
 struct Deriv64 {
@@ -519,11 +522,13 @@ struct Tracer32 {
     float rh, rl, th_h, th_l, ph_h, ph_l;  // positions as compensated pairs (value = hi + lo)
     float pr, pth, pt, pphi;
     float tau, drift, H0;
+    float leave;  // a step that ends beyond this radius moving out answers kLeft (the escape radius, or r_far)
     int steps, brick, vi;
     uint32_t out_idx;
 
     __device__ __forceinline__ void init(const ViewDev &v, int view, int px, int py, int64_t out_index) {
         const CameraRay c = camera_ray(v, px, py);
+        leave = (float)v.escape_radius;
         split(v.r_obs, rh, rl);
         split(v.theta_obs, th_h, th_l);
         double p0 = fmod(v.phi_obs, kTwoPi);
@@ -608,9 +613,10 @@ struct Tracer32 {
             Deriv32 k2;
             rhs32(fmaf(hh, k1.r, r0), fmaf(hh, k1.r, x0), s, c, fmaf(hh, k1.pr, pr), fmaf(hh, k1.pth, pth), pt, pphi,
                   C.a, C.a2, C.dpm, k2);
-            dr = h * k2.r;
-            const float dth = h * k2.th;
-            dph = h * k2.ph;
+            // rounded products: the compensated sums below must not contract with them (far_steps takes the same steps)
+            dr = __fmul_rn(h, k2.r);
+            const float dth = __fmul_rn(h, k2.th);
+            dph = __fmul_rn(h, k2.ph);
             const float prn = fmaf(h, k2.pr, pr), pthn = fmaf(h, k2.pth, pth);
             // An FP32 overflow here (a ray flung off the pole or out of the
             // horizon reaches momenta of 1e30 and more, whose squares FP64 still
@@ -748,7 +754,10 @@ struct Tracer32 {
         if (!finite) return BHN_RAY_INVALID;
         if (tau >= C.max_tau) return BHN_RAY_OPAQUE;
         if ((rh - C.rcap_h) + (rl - C.rcap_l) <= 0.0f) return BHN_RAY_CAPTURED;
-        if (rh > C.esc && dr > 0.0f) return BHN_RAY_ESCAPED;
+        if (rh > leave && dr > 0.0f) {
+            if (rh > C.esc) return BHN_RAY_ESCAPED;
+            if (steps < C.max_steps) return kLeft;
+        }
         if (steps >= C.max_steps) return BHN_RAY_MAX_STEPS;
         return -1;
     }
@@ -938,6 +947,10 @@ struct Tracer64 {
     }
 };
 
+}  // namespace bhn
+#include "bhn_far.cuh"
+namespace bhn {
+
 template <class T> struct RecordOf;
 template <> struct RecordOf<Tracer32> { using type = float4; };
 template <> struct RecordOf<Tracer64> { using type = double2; };
@@ -989,7 +1002,8 @@ __global__ void __launch_bounds__(256, MINB) render_kernel(const RenderParams P)
         c.esc = (float)v.escape_radius;
         c.r_guard = (v.flags & BHN_VIEW_HORIZON_GUARD) ? (float)fmin(v.r_photon, T.gr[0]) : 0.0f;
         c.r_near = (float)(v.r_plus + kNearHorizon);
-        c.pad = 0.0f;
+        // the factor covers the midpoint's and the knots' FP32 rounding
+        c.r_far = fmaxf(fmaxf(T.grf[P.nr - 1], c.r_near), fmaxf(c.r_guard, c.rcap_h)) * 1.0001f + 1.0e-3f;
         c.max_steps = v.max_steps;
         c.pad1 = c.pad2 = c.pad3 = 0;
         sconst[i] = c;
@@ -1003,6 +1017,54 @@ __global__ void __launch_bounds__(256, MINB) render_kernel(const RenderParams P)
     const unsigned lt_mask = (1u << lane) - 1u;
     Tracer tr;
     bool alive = false, exhausted = BATCH;
+
+    // One ray's results and the block's totals.
+    auto finish_ray = [&](Tracer &t, int st, const StepConst &C) {
+        t.finish(P.out, st, C, P.views);
+        const float d = t.drift_f();
+        atomicAdd(&bc->steps, (unsigned long long)t.steps);
+        atomicAdd(&bc->brick, (unsigned long long)t.brick);
+        atomicAdd(&bc->rays, 1u);
+        atomicAdd(&bc->status[st], 1u);
+        atomicMax(reinterpret_cast<unsigned int *>(&bc->max_drift), __float_as_uint(d));
+        if (st == BHN_RAY_ESCAPED)
+            atomicMax(reinterpret_cast<unsigned int *>(&bc->max_drift_escaped), __float_as_uint(d));
+        if (P.ray_steps) P.ray_steps[t.out_idx] = t.steps;
+        if (P.ray_status) P.ray_status[t.out_idx] = (uint8_t)st;
+        if (P.ray_drift) P.ray_drift[t.out_idx] = d;
+    };
+    // no step is taken: the reference returns a zero Stokes vector
+    auto skip_ray = [&](const ViewDev &v, int64_t out_idx) {
+        Tracer::write_zero(P.out, out_idx);
+        const int zst = v.valid ? BHN_RAY_MAX_STEPS : BHN_RAY_INVALID;
+        atomicAdd(&bc->rays, 1u);
+        atomicAdd(&bc->status[zst], 1u);
+        if (P.ray_steps) P.ray_steps[out_idx] = 0;
+        if (P.ray_status) P.ray_status[out_idx] = (uint8_t)zst;
+        if (P.ray_drift) P.ray_drift[out_idx] = 0.0f;
+    };
+    // The FP32 steps in a tight inner loop; an island step leaves it for the
+    // out-of-line FP64 step and comes back.
+    auto trace = [&](Tracer &t, const StepConst &C) -> int {
+        int st;
+        for (;;) {
+            if constexpr (Tracer::kIslands) far_steps(t, C);
+            do {
+                st = t.step(C, T, rec, P.nr, P.nt, P.np, P.views);
+            } while (st == -1);
+            if constexpr (Tracer::kIslands) {
+                if (st == kNeedFp64) st = t.step64(C, T, rec, P.nr, P.nt, P.np, P.views);
+                if (st == kLeft) {
+                    t.leave = C.esc;
+                    continue;
+                }
+                if (st != -1) break;
+            } else {
+                break;
+            }
+        }
+        return st;
+    };
 
     // Batch mode (refill_min = 32): a warp takes 32 consecutive ray slots with one
     // atomic and every lane traces its ray to the end in a tight loop; the warp
@@ -1023,41 +1085,10 @@ __global__ void __launch_bounds__(256, MINB) render_kernel(const RenderParams P)
             if (v.valid && v.max_steps > 0) {
                 tr.init(v, vi, px.px, px.py, px.out_idx);
                 const StepConst &C = sconst[vi];
-                int st;
-                // the FP32 steps in a tight inner loop; an island step leaves it
-                // for the out-of-line FP64 step and comes back
-                for (;;) {
-                    do {
-                        st = tr.step(C, T, rec, P.nr, P.nt, P.np, P.views);
-                    } while (st == -1);
-                    if constexpr (Tracer::kIslands) {
-                        if (st != kNeedFp64) break;
-                        st = tr.step64(C, T, rec, P.nr, P.nt, P.np, P.views);
-                        if (st != -1) break;
-                    } else {
-                        break;
-                    }
-                }
-                tr.finish(P.out, st, C, P.views);
-                const float d = tr.drift_f();
-                atomicAdd(&bc->steps, (unsigned long long)tr.steps);
-                atomicAdd(&bc->brick, (unsigned long long)tr.brick);
-                atomicAdd(&bc->rays, 1u);
-                atomicAdd(&bc->status[st], 1u);
-                atomicMax(reinterpret_cast<unsigned int *>(&bc->max_drift), __float_as_uint(d));
-                if (st == BHN_RAY_ESCAPED)
-                    atomicMax(reinterpret_cast<unsigned int *>(&bc->max_drift_escaped), __float_as_uint(d));
-                if (P.ray_steps) P.ray_steps[tr.out_idx] = tr.steps;
-                if (P.ray_status) P.ray_status[tr.out_idx] = (uint8_t)st;
-                if (P.ray_drift) P.ray_drift[tr.out_idx] = d;
+                if constexpr (Tracer::kIslands) tr.leave = fminf(C.r_far, C.esc);
+                finish_ray(tr, trace(tr, C), C);
             } else {
-                Tracer::write_zero(P.out, px.out_idx);
-                const int zst = v.valid ? BHN_RAY_MAX_STEPS : BHN_RAY_INVALID;
-                atomicAdd(&bc->rays, 1u);
-                atomicAdd(&bc->status[zst], 1u);
-                if (P.ray_steps) P.ray_steps[px.out_idx] = 0;
-                if (P.ray_status) P.ray_status[px.out_idx] = (uint8_t)zst;
-                if (P.ray_drift) P.ray_drift[px.out_idx] = 0.0f;
+                skip_ray(v, px.out_idx);
             }
         }
         __syncwarp();
@@ -1087,14 +1118,7 @@ __global__ void __launch_bounds__(256, MINB) render_kernel(const RenderParams P)
                         tr.init(v, vi, px.px, px.py, px.out_idx);
                         alive = true;
                     } else {
-                        // no step is taken: the reference returns a zero Stokes vector
-                        Tracer::write_zero(P.out, px.out_idx);
-                        const int zst = v.valid ? BHN_RAY_MAX_STEPS : BHN_RAY_INVALID;
-                        atomicAdd(&bc->rays, 1u);
-                        atomicAdd(&bc->status[zst], 1u);
-                        if (P.ray_steps) P.ray_steps[px.out_idx] = 0;
-                        if (P.ray_status) P.ray_status[px.out_idx] = (uint8_t)zst;
-                        if (P.ray_drift) P.ray_drift[px.out_idx] = 0.0f;
+                        skip_ray(v, px.out_idx);
                     }
                 }
             }
@@ -1110,18 +1134,7 @@ __global__ void __launch_bounds__(256, MINB) render_kernel(const RenderParams P)
                 if (st == kNeedFp64) st = tr.step64(C, T, rec, P.nr, P.nt, P.np, P.views);
             }
             if (st >= 0) {
-                tr.finish(P.out, st, C, P.views);
-                const float d = tr.drift_f();
-                atomicAdd(&bc->steps, (unsigned long long)tr.steps);
-                atomicAdd(&bc->brick, (unsigned long long)tr.brick);
-                atomicAdd(&bc->rays, 1u);
-                atomicAdd(&bc->status[st], 1u);
-                atomicMax(reinterpret_cast<unsigned int *>(&bc->max_drift), __float_as_uint(d));
-                if (st == BHN_RAY_ESCAPED)
-                    atomicMax(reinterpret_cast<unsigned int *>(&bc->max_drift_escaped), __float_as_uint(d));
-                if (P.ray_steps) P.ray_steps[tr.out_idx] = tr.steps;
-                if (P.ray_status) P.ray_status[tr.out_idx] = (uint8_t)st;
-                if (P.ray_drift) P.ray_drift[tr.out_idx] = d;
+                finish_ray(tr, st, C);
                 alive = false;
             }
         }
