@@ -138,10 +138,16 @@ __global__ void __launch_bounds__(128, 4) brick_trace_kernel(const BrickTracePar
 // each scheduler idle while the warp waits on its own dependent FP64 chain:
 // the RK4 steps and, for every step inside the brick, the sample and Stokes
 // step.  Here a block of two warps takes 32 rays: warp 0 integrates the
-// geodesics and publishes each accepted state through a ring of kRing slots in
+// geodesics and publishes the accepted states through a ring of kRing slots in
 // shared memory; warp 1 takes the segments from it -- sample, Stokes step,
 // optical depth -- and reports the cutoff back.  Same arithmetic, same image.
-constexpr int kRing = 32;
+//
+// What bounds it is warp 0's chain of RK4 steps: 160 x 90 takes 3.40 ms with
+// warp 1's work left out.  The states go over in groups of kBatch: a barrier
+// phase per state, with its wait, its arrival and the read of the cutoff
+// between two steps, cost 4.38 ms; 4 states a phase 4.13, 8 states 4.08 (the
+// ring is the same 32 states, so warp 0 runs no further ahead of a cutoff).
+constexpr int kBatch = 8, kGroups = 4, kRing = kBatch * kGroups;  // states per barrier phase; phases in flight
 #ifndef BHN_PAIR_WARPS_PER_SM
 #define BHN_PAIR_WARPS_PER_SM 4
 #endif
@@ -150,11 +156,11 @@ constexpr long long kWaitCycles = 4000000000LL;  // ~2 s: a wait that long is a 
 enum : int { kSlotDead = 0, kSlotLive = 1, kSlotEnd = 2 };
 
 struct PairRing {
-    double st[kRing][3][32];          // r, theta, phi after step j, at slot j % kRing
-    int flag[kRing][32];              // kSlot*
-    unsigned long long full[kRing];   // mbarriers: 32 arrivals (warp 0) per fill
-    unsigned long long empty[kRing];  // 32 arrivals (warp 1) per drain
-    int stop_step[32];                // warp 1 -> 0: step whose segment reached the cutoff (0: none)
+    double st[kRing][3][32];            // r, theta, phi after step j, at slot j % kRing
+    int flag[kRing][32];                // kSlot*
+    unsigned long long full[kGroups];   // mbarriers: 32 arrivals (warp 0) per filled group of kBatch slots
+    unsigned long long empty[kGroups];  // 32 arrivals (warp 1) per drained group
+    int stop_step[32];                  // warp 1 -> 0: step whose segment reached the cutoff (0: none)
     int end_steps[32], end_status[32];  // warp 0 -> 1, written before the end slot
 };
 
@@ -190,7 +196,7 @@ __global__ void __launch_bounds__(64) brick_trace_pair_kernel(const BrickTracePa
     const int64_t r = (int64_t)blockIdx.x * 32 + lane;
     const bool in_image = r < rays;
     if (threadIdx.x == 0) {
-        for (int k = 0; k < kRing; ++k) {
+        for (int k = 0; k < kGroups; ++k) {
             mbar_init(&R.full[k], 32);
             mbar_init(&R.empty[k], 32);
         }
@@ -202,7 +208,7 @@ __global__ void __launch_bounds__(64) brick_trace_pair_kernel(const BrickTracePa
 
     if (warp == 0) {  // ------------------------------------------- geodesics
         double y[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, pt = 0.0, pphi = 0.0;
-        const double a = v.a;
+        const double a = v.a, r_capture = v.r_capture;
         if (traced) {
             const CameraRay cam = camera_ray(v, px, py);
             y[0] = v.r_obs;
@@ -214,86 +220,96 @@ __global__ void __launch_bounds__(64) brick_trace_pair_kernel(const BrickTracePa
             pphi = cam.pphi;
         }
         const double r_edge = P.full_trace ? INFINITY : fmax(P.rg[0], P.rg[P.nr - 1]);
-        bool alive = traced;
+        bool alive = traced, more = true;
         int steps = 0, status = traced ? BHN_RAY_MAX_STEPS : BHN_RAY_INVALID;
         double prev_r = y[0];
-        // slot j: the states after step j (j = 0: the camera), then one end slot
-        auto publish = [&](int jj, int flag) -> bool {
-            const int k = jj % kRing, f = jj / kRing;
-            if (f > 0 && !__all_sync(0xffffffffu, mbar_wait(&R.empty[k], (f - 1) & 1))) return false;  // whole warp
-            R.st[k][0][lane] = y[0];
-            R.st[k][1][lane] = y[1];
-            R.st[k][2][lane] = y[2];
-            R.flag[k][lane] = flag;
-            mbar_arrive(&R.full[k]);
-            return true;
-        };
-        if (!publish(0, traced ? kSlotLive : kSlotDead)) {
-            atomicOr(error_flags, 1u);
-            return;
-        }
-        int i = 1;
-        for (;; ++i) {
-            // step i (kerr.py:355-378), while the transfer has not reached its cutoff
-            const bool live = alive && i <= P.max_steps && *((volatile int *)&R.stop_step[lane]) == 0;
-            if (!__any_sync(0xffffffffu, live)) break;
-            int flag = kSlotDead;
-            if (live) {
-                double yn[5];
-                rk4_state(y, P.step, a, pt, pphi, yn);
-                steps = i;
-                if (!(isfinite(yn[0]) && isfinite(yn[1]) && isfinite(yn[2]) && isfinite(yn[3]) && isfinite(yn[4]))) {
-                    status = BHN_RAY_INVALID;  // kerr.py:364-366: the state is not stored
-                    alive = false;
-                } else {
-                    for (int q = 0; q < 5; ++q) y[q] = yn[q];
-                    flag = kSlotLive;
-                    if (y[0] <= v.r_capture) {
-                        status = BHN_RAY_CAPTURED;
-                        alive = false;
-                    } else if (y[0] > P.escape_radius && y[0] > prev_r) {
-                        status = BHN_RAY_ESCAPED;
-                        alive = false;
-                    } else if (y[0] > r_edge && outbound_for_good(y[0], y[1], y[3], y[4], pt, pphi, a)) {
-                        status = BHN_RAY_OUTBOUND;  // no later segment is sampled
-                        alive = false;
-                    }
-                    prev_r = y[0];
-                }
-            }
-            if (!publish(i, flag)) {
+        // slot j: the states after step j (j = 0: the camera), then one end slot; a group's slots are published together
+        for (int i = 0; more; i += kBatch) {
+            const int g = i / kBatch % kGroups, f = i / kRing;
+            if (f > 0 && !__all_sync(0xffffffffu, mbar_wait(&R.empty[g], (f - 1) & 1))) {  // whole warp
                 atomicOr(error_flags, 1u);
                 return;
             }
+            // while the transfer has not reached its cutoff (it may run up to a ring of steps behind: those are dropped)
+            if (*((volatile int *)&R.stop_step[lane]) != 0) alive = false;
+#pragma unroll 1
+            for (int b = 0; b < kBatch; ++b) {
+                const int j = i + b, slot = g * kBatch + b;
+                int flag = kSlotDead;
+                if (j == 0) {
+                    flag = traced ? kSlotLive : kSlotDead;
+                } else {
+                    const bool live = alive && j <= P.max_steps;
+                    if (!__any_sync(0xffffffffu, live)) {
+                        R.end_steps[lane] = steps;
+                        R.end_status[lane] = status;
+                        R.flag[slot][lane] = kSlotEnd;
+                        more = false;
+                        break;
+                    }
+                    if (live) {  // step j (kerr.py:355-378)
+                        double yn[5];
+                        rk4_state(y, P.step, a, pt, pphi, yn);
+                        steps = j;
+                        if (!(isfinite(yn[0]) && isfinite(yn[1]) && isfinite(yn[2]) && isfinite(yn[3]) &&
+                              isfinite(yn[4]))) {
+                            status = BHN_RAY_INVALID;  // kerr.py:364-366: the state is not stored
+                            alive = false;
+                        } else {
+                            for (int q = 0; q < 5; ++q) y[q] = yn[q];
+                            flag = kSlotLive;
+                            if (y[0] <= r_capture) {
+                                status = BHN_RAY_CAPTURED;
+                                alive = false;
+                            } else if (y[0] > P.escape_radius && y[0] > prev_r) {
+                                status = BHN_RAY_ESCAPED;
+                                alive = false;
+                            } else if (y[0] > r_edge && outbound_for_good(y[0], y[1], y[3], y[4], pt, pphi, a)) {
+                                status = BHN_RAY_OUTBOUND;  // no later segment is sampled
+                                alive = false;
+                            }
+                            prev_r = y[0];
+                        }
+                    }
+                }
+                R.st[slot][0][lane] = y[0];
+                R.st[slot][1][lane] = y[1];
+                R.st[slot][2][lane] = y[2];
+                R.flag[slot][lane] = flag;
+            }
+            mbar_arrive(&R.full[g]);
         }
-        R.end_steps[lane] = steps;
-        R.end_status[lane] = status;
-        if (!publish(i, kSlotEnd)) atomicOr(error_flags, 1u);  // the end slot carries end_steps / end_status
     } else {  // ------------------------------------------------- transfer
         const AxisHints hints = shared_hints;
         double S[4] = {0.0, 0.0, 0.0, 0.0}, prev[3] = {0.0, 0.0, 0.0}, tau = 0.0;
         int sampled = 0, stop_at = 0;
-        bool ok = true;
-        for (int j = 0;; ++j) {
-            const int k = j % kRing, f = j / kRing;
-            if (!__all_sync(0xffffffffu, mbar_wait(&R.full[k], f & 1))) {  // the whole warp gives up together
+        bool ok = true, more = true;
+        for (int i = 0; more; i += kBatch) {
+            const int g = i / kBatch % kGroups, f = i / kRing;
+            if (!__all_sync(0xffffffffu, mbar_wait(&R.full[g], f & 1))) {  // the whole warp gives up together
                 atomicOr(error_flags, 1u);
                 ok = false;
                 break;
             }
-            const double cur[3] = {R.st[k][0][lane], R.st[k][1][lane], R.st[k][2][lane]};
-            const int flag = R.flag[k][lane];
-            mbar_arrive(&R.empty[k]);
-            if (flag == kSlotEnd) break;
-            if (flag == kSlotLive) {
-                if (j > 0 && stop_at == 0 && transfer_segment<Layout>(P, hints, prev, cur, S, tau, sampled)) {
-                    stop_at = j;  // the cutoff (accelerated_renderer.py:123-125): nothing later changes the image
-                    R.stop_step[lane] = j;
+#pragma unroll 1
+            for (int b = 0; b < kBatch; ++b) {
+                const int j = i + b, slot = g * kBatch + b, flag = R.flag[slot][lane];
+                if (flag == kSlotEnd) {  // every lane's, in the same slot
+                    more = false;
+                    break;
                 }
-                prev[0] = cur[0];
-                prev[1] = cur[1];
-                prev[2] = cur[2];
+                if (flag == kSlotLive) {
+                    const double cur[3] = {R.st[slot][0][lane], R.st[slot][1][lane], R.st[slot][2][lane]};
+                    if (j > 0 && stop_at == 0 && transfer_segment<Layout>(P, hints, prev, cur, S, tau, sampled)) {
+                        stop_at = j;  // the cutoff (accelerated_renderer.py:123-125): nothing later changes the image
+                        R.stop_step[lane] = j;
+                    }
+                    prev[0] = cur[0];
+                    prev[1] = cur[1];
+                    prev[2] = cur[2];
+                }
             }
+            mbar_arrive(&R.empty[g]);
         }
         if (in_image) {
             const int64_t o = v.out_offset + r;
@@ -350,7 +366,7 @@ extern "C" int bhn_brick_trace_render(const void *coeffs, const double *r_grid, 
     P.diag = diag;
     // Two warps per 32 rays while the one-warp form would leave schedulers idle (at most one ray
     // warp per scheduler, 4 per SM); above that the one-warp form wins (200 x 112, 4.7 ray warps
-    // per SM: 6.52 against 7.17 ms; 256 x 144, 7.8 per SM: even; 160 x 90, 3 per SM: 4.33 against 6.3).
+    // per SM: 6.52 against 7.17 ms; 256 x 144, 7.8 per SM: even; 160 x 90, 3 per SM: 4.08 against 6.3).
     const int64_t warps = (rays + 31) / 32;
     if (warps <= (int64_t)kPairWarpsPerSm * sm_count_current_device()) {
         unsigned *flags = &reinterpret_cast<QueueState *>(static_cast<unsigned char *>(scratch) +
