@@ -30,12 +30,13 @@ static int frames_per_warp(int64_t n, int sms) {
 
 // Six 128-thread blocks per SM (80 registers): 30,011 Hybrid frames took 188
 // us against 242 at five and 193 at seven and eight, before the power law's
-// nodes were grouped.  Now 108 us and 51 us for the tables (728 us with one
-// frame per warp and two exp() per node and pitch angle), 2.7 ns a frame at a
-// million and more (22.6); 1,450 instructions a frame, of them about 40 % the
-// thermal nodes' exp, log and sqrt, and 30 L1 wavefronts a row chunk: neither
-// the issue slots nor the L1 pipe is more than two thirds busy, fixed FP64
-// latencies and the shared-memory round trip of add_nodes fill the rest.
+// nodes were grouped.  Now 100 us and 35 us for the tables (728 us with one
+// frame per warp and two exp() per node and pitch angle), 2.5 ns a frame at a
+// million and more (22.6).  Leaving out the row lookups takes three quarters
+// of it, cheap stand-ins for log or exp 9 % each; the issue slots are two
+// thirds busy, fixed FP64 latencies and the shared-memory round trip of
+// add_nodes fill the rest.  Two chunks of nodes per exchange, to overlap
+// those, were slower (116 us; 125 at four blocks without spills).
 struct PrecomputeParams {
     Model M;
     double nu;
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(128, 6) frame_coefficients_kernel(const __grid
 constexpr int kSeries = 12;  // Taylor terms before economisation
 
 // Terms first, first + stride, ... of a row's Taylor series (F and G) about
-// its centre, in units of the half width h.  A term sees the table segment at
+// its centre, in units of the half width h, each times its degree's factorial.  A term sees the table segment at
 // its x (numpy.interp: constant past either end of the knots).
 __host__ __device__ inline void row_series(const KernelTable &K, const SumPlan &P, double centre, double h, int first,
                                            int stride, double aF[kSeries], double aG[kSeries]) {
@@ -146,16 +147,16 @@ __host__ __device__ inline void row_series(const KernelTable &K, const SumPlan &
             sF = sG = 0.0;
         }
         double uF = P.weight[t] * exp(vF), uG = P.weight[t] * exp(vG);
-        for (int d = 0; d < kSeries; ++d) {
+        for (int d = 0; d < kSeries; ++d) {  // moments; the factorials follow the sum
             aF[d] += uF;
             aG[d] += uG;
-            uF *= sF * (1.0 / (d + 1));
-            uG *= sG * (1.0 / (d + 1));
+            uF *= sF;
+            uG *= sG;
         }
     }
 }
 
-// The series economised to degree 7 (v^n -> v^n - T_n(v) / 2^(n-1), n = 11 .. 8,
+// The series of row_series economised to degree 7 (v^n -> v^n - T_n(v) / 2^(n-1), n = 11 .. 8,
 // v = z / h) and scaled to powers of z.
 __host__ __device__ inline void row_coefficients(double a[kSeries], double h, double co[8]) {
     // Chebyshev polynomials T_11 .. T_8 below their leading terms
@@ -163,6 +164,10 @@ __host__ __device__ inline void row_coefficients(double a[kSeries], double h, do
     const double t10[5] = {-1.0, 50.0, -400.0, 1120.0, -1280.0};     // 1, v^2 .. v^8
     const double t9[4] = {9.0, -120.0, 432.0, -576.0};
     const double t8[4] = {1.0, -32.0, 160.0, -256.0};
+    const double inverse[kSeries] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040, 1.0 / 40320,
+                                     1.0 / 362880, 1.0 / 3628800, 1.0 / 39916800};  // factorials
+#pragma unroll
+    for (int d = 2; d < kSeries; ++d) a[d] *= inverse[d];
     for (int d = 0; d < 5; ++d) a[2 * d + 1] -= a[11] * t11[d] * (1.0 / 1024.0);
     for (int d = 0; d < 5; ++d) a[2 * d] -= a[10] * t10[d] * (1.0 / 512.0);
     for (int d = 0; d < 4; ++d) a[2 * d + 1] -= a[9] * t9[d] * (1.0 / 256.0);
@@ -196,10 +201,14 @@ struct TableParams {
     double p, gamma_min, gamma_max;
 };
 
-// The tables of one call: four lanes per row, each a quarter of the sum's
-// terms; the last block makes the power law's nodes.  Tens of thousands of rows
-// and no reuse: bound by its exponentials (two per term).
-constexpr int kRowLanes = 4;
+// The tables of one call: two lanes per row, each half of the sum's terms and
+// then one of the two kernels' coefficients; the last block makes the power
+// law's nodes.  Tens of thousands of rows and no reuse: bound by the FP64 work
+// of a term (two exponentials, 24 moments) and a row (economisation).  The
+// default Hybrid model's 39,892 rows take 35 us (four lanes 43, with two more
+// rounds of 24 shuffles); 51 us with a product more per moment and with the
+// rows past the far tail, a fifth of them, which no lookup reaches.
+constexpr int kRowLanes = 2;
 __global__ void __launch_bounds__(128) sum_table_kernel(const __grid_constant__ TableParams P) {
     __shared__ KernelTable K;
     if (blockIdx.x == gridDim.x - 1) {
@@ -384,10 +393,10 @@ void pitch_terms(int n, SumPlan &ps) {
 
 // The pieces that the table knots seen through a sum's terms cut a cell into
 // (wide gaps split: at most a quarter of a cell, or twice the mean) and every
-// cell's split into rows.
+// cell's split into rows.  The cells end with the far tail: no lookup passes it.
 int cells_of(double y0, double shift_max) {
     const KernelTable &K = host_table();
-    return (int)std::floor((K.lx[kTable - 1] + shift_max - y0) * ((kTable - 1) / (K.lx[kTable - 1] - K.lx[0])) + 0.5) + 2;
+    return (int)std::floor((K.lx_tail + shift_max - y0) * ((kTable - 1) / (K.lx[kTable - 1] - K.lx[0])) + 0.5) + 2;
 }
 void make_plan(SumPlan &P) {
     const KernelTable &K = host_table();

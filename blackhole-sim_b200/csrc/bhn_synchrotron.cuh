@@ -129,13 +129,13 @@ struct PieceSmem {
     float inv_width[kMaxPieces];
     int first[kBins], cell[kMaxCells];
 };
-// One warp's exchange between the nodes (a lane each) and the row loads (eight
-// lanes a row): per node its row and its weight times the powers of z.  A
-// stride of 36 doubles puts the eight powers of four neighbouring nodes on
-// distinct banks.
-constexpr int kPowStride = 36;
+// One warp's exchange between the nodes (a lane each) and the row loads (four
+// lanes a row): per node its row and its weight times the powers of z.  Node n
+// keeps powers 2 q and 2 q + 1 in pair 4 n + (q ^ (n / 2 & 3)), and its row
+// at 4 (n % 8) + n / 8: the eight lanes of one 16-byte access, eight nodes
+// writing or two being read, then lie on distinct banks.
 struct __align__(16) NodeSmem {
-    double pow[8 * kPowStride];
+    double2 pow[4 * 32];
     int row[32];
 };
 constexpr int kSynchWarps = 4;  // warps per block of the evaluation kernels
@@ -150,11 +150,20 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// 2^n, -1022 <= n <= 1023
+__host__ __device__ __forceinline__ double pow2(int n) {
+#ifdef __CUDA_ARCH__
+    return __hiloint2double((n + 1023) << 20, 0);
+#else
+    return std::ldexp(1.0, n);
+#endif
+}
+
 // L at the centre of row `sub` of 2^split in the piece [left, left + width) of cell c (table build and lookup alike).
 __host__ __device__ __forceinline__ double row_centre(double y0, double delta, double c, double left, double width,
                                                       int split, int sub) {
     double at = 0.5;
-    if (split) at = ((double)sub + 0.5) / (double)(1 << split);  // exact
+    if (split) at = ((double)sub + 0.5) * pow2(-split);  // exact
     return fma(c + fma(at, width, left), delta, y0);
 }
 
@@ -189,6 +198,11 @@ __device__ __forceinline__ int sum_row(const SumTable &T, const PieceSmem &S, do
     return (cell >> 4) + (k << split) + sub;
 }
 
+// Four doubles of read-only global memory in one load (32-byte aligned).
+__device__ __forceinline__ void load_32_bytes(const void *p, double (&v)[4]) {
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+
 struct Integrals {
     double norm, I, Q;   // sum c_i f_i, sum c_i f_i sum_m W_m F, sum c_i f_i sum_m W_m G
 };
@@ -196,10 +210,12 @@ struct Integrals {
 // Adds w (F, G)(L) of one node per lane to the lanes' partial sums.  The rows
 // lie anywhere in a table of a megabyte, so a lane reading its own row would
 // touch 32 cache lines with every load (8 loads: 256 L1 wavefronts, which
-// bound the kernel at 92 % of the L1 pipe, 24 ms for 2.46M cells); instead eight
-// lanes read a row together (one line), each multiplying the coefficients of
-// its degree by the node's w z^degree from shared memory, and the sum over the
-// degrees falls to the reduction that sums the nodes: 73 wavefronts, 13.7 ms.
+// bound the kernel at 92 % of the L1 pipe, 24 ms for 2.46M cells); instead four
+// lanes read a row together (one line, 32 bytes each), each multiplying the
+// coefficients of its two degrees by the node's w z^degree from shared memory,
+// and the sum over the degrees falls to the reduction that sums the nodes:
+// 13.7 ms with eight lanes and 16 bytes.  The wide loads and paired powers
+// halve the exchange's instructions: 30,011 Hybrid frames 106.6 -> 100.1 us.
 // A node whose smallest x (the pitch with the largest sin) already lies in
 // the table's far tail adds terms below kTailValue times the pitch weights
 // (< 1e-270): nothing a cell that emits can resolve.  Skipping it leaves such
@@ -213,22 +229,29 @@ __device__ __forceinline__ void add_nodes(const SumTable &T, const PieceSmem &S,
     double z = 0.0, p = 0.0;
     int row = 0;
     if (live) {
-        row = 8 * sum_row(T, S, L, z);
+        row = sum_row(T, S, L, z);
         p = w;
     }
-    X.row[lane] = row;
+    X.row[4 * (lane & 7) + (lane >> 3)] = row;
+    const double zz = z * z;
+    double p1 = p * z;
 #pragma unroll
-    for (int d = 0; d < 8; ++d, p *= z) X.pow[d * kPowStride + lane] = p;
+    for (int q = 0; q < 4; ++q, p *= zz, p1 *= zz) X.pow[4 * lane + (q ^ ((lane >> 1) & 3))] = make_double2(p, p1);
     __syncwarp();
-    const int d = lane & 7, g = lane >> 3;
-    const double2 *coefficient = T.rows + d;
-    const double *power = X.pow + d * kPowStride + g;
+    const int q = lane & 3, g = lane >> 2;  // rows g, g + 8, g + 16, g + 24; degrees 2 q and 2 q + 1
+    const int4 four = *reinterpret_cast<const int4 *>(X.row + 4 * g);
+    const int rows[4] = {four.x, four.y, four.z, four.w};
+    const double2 *power = X.pow + 4 * g + (q ^ ((g >> 1) & 3));
+    const double2 *coefficient = T.rows + 2 * q;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const double2 c = __ldg(coefficient + X.row[4 * j + g]);
-        const double q = power[4 * j];
-        acc.I = fma(q, c.x, acc.I);
-        acc.Q = fma(q, c.y, acc.Q);
+    for (int j = 0; j < 4; ++j) {
+        const double2 v = power[32 * j];
+        double c[4];
+        load_32_bytes(coefficient + 8 * rows[j], c);
+        acc.I = fma(v.x, c[0], acc.I);
+        acc.Q = fma(v.x, c[1], acc.Q);
+        acc.I = fma(v.y, c[2], acc.I);
+        acc.Q = fma(v.y, c[3], acc.Q);
     }
     __syncwarp();
 }
