@@ -113,15 +113,22 @@ __global__ void __launch_bounds__(256) cell_key_kernel(const double *__restrict_
 // ORDERED: points in cell order, the cell decoded from the sorted key; a
 // point's coordinates then lie anywhere, so the next batch's are loaded before
 // this batch's corners.
-// 12.6M points in cell order through a 738 MB brick: 985 us (1,590 with a lane
-// per point), 100,003 through 11 MB in input order: 13 us (31).  Half of it is
-// the corners (L1 wavefronts 70 % busy, FP64 26 %: the reference's separately
-// rounded lerps), a quarter the scattered 24-byte reads and 32-byte writes of
-// the cell order.  One 1,024-thread block per SM on consecutive points keeps
+// 12.6M points in cell order through a 738 MB brick: 917 us (1,590 with a lane
+// per point), 100,003 through 11 MB in input order: 13 us (31).  Two thirds of
+// it is the corners (L1 wavefronts 75 % busy, FP64 26 %: the reference's
+// separately rounded lerps), the rest the scattered reads and writes of the
+// cell order, where every lane's access is a wavefront of its own: a point's
+// 24 bytes in two loads and its 32 in one store, where the arrays' alignment
+// allows, instead of three and two (985 us; the loads alone give 992, the store
+// alone 941).  One 1,024-thread block per SM on consecutive points keeps
 // the theta rows that neighbouring points share in L1: 1,068 us at 128-thread
 // blocks, 1,026 at 256, 1,008 at 512; a contiguous share of the points per
 // block instead 1,211 (every SM then reads its own r slabs from memory); all
-// eleven channel steps unrolled 1,407 (122 registers, half the warps).
+// eleven channel steps unrolled 1,407 (122 registers, half the warps).  Corners
+// kept in registers from point to point of a cell or its phi neighbour save
+// two thirds of the corner loads but wait for them in turn (22 lanes on runs of
+// 16 points: 1,056; pairs of points: 961); the next batch's corners prefetched
+// into L2: 1,003.
 struct __align__(16) Place {  // a point's cells (r0, theta0, phi0) and (r0, theta0, phi1) and its weights
     double wr, wt, wp;
     uint32_t cell0, cell1;
@@ -130,6 +137,11 @@ struct WarpPoints {
     Place place[32];
     double value[32 * 11];
 };
+// Four doubles in one 32-byte store (32-byte aligned).
+__device__ __forceinline__ void store_32_bytes(double *p, const double (&v)[4]) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]) : "memory");
+}
+
 template <bool STEP, bool ORDERED>
 __global__ void __launch_bounds__(kSampleThreads, kSampleBlocks) sample_points_kernel(const SamplePoints P) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -143,6 +155,8 @@ __global__ void __launch_bounds__(kSampleThreads, kSampleBlocks) sample_points_k
     int64_t base = (int64_t)blockIdx.x * blockDim.x + 32 * warp;
     uint32_t next_i = 0, next_key = P.invalid_key;
     double nr_ = 0.0, nt_ = 0.0, np_ = 0.0;
+    const bool aligned16 = (reinterpret_cast<uintptr_t>(P.pts) & 15) == 0;  // else three 8-byte reads
+    const bool aligned32 = (reinterpret_cast<uintptr_t>(P.out) & 31) == 0;  // else two 16-byte writes
     auto fetch = [&](int64_t k) {  // point k of the order (k < n) into next_*
         if (k >= P.n) return;
         int64_t i = k;
@@ -151,9 +165,19 @@ __global__ void __launch_bounds__(kSampleThreads, kSampleBlocks) sample_points_k
             next_key = __ldcs(P.keys + k);
             i = next_i;
         }
-        nr_ = P.pts[3 * i];
-        nt_ = P.pts[3 * i + 1];
-        np_ = P.pts[3 * i + 2];
+        if (ORDERED && aligned16) {  // an even point starts on 16 bytes, an odd one 8 before
+            const bool odd = i & 1;
+            const double *q = P.pts + 3 * i;
+            const double2 two = *reinterpret_cast<const double2 *>(q + odd);
+            const double one = q[odd ? 0 : 2];
+            nr_ = odd ? one : two.x;
+            nt_ = odd ? two.x : two.y;
+            np_ = odd ? two.y : one;
+        } else {
+            nr_ = P.pts[3 * i];
+            nt_ = P.pts[3 * i + 1];
+            np_ = P.pts[3 * i + 2];
+        }
     };
     fetch(base + lane);
     for (; base < P.n; base += step) {
@@ -228,8 +252,12 @@ __global__ void __launch_bounds__(kSampleThreads, kSampleBlocks) sample_points_k
                 } else if (P.policy != BHN_POLICY_INITIAL) {
                     s[0] = s[1] = s[2] = s[3] = __longlong_as_double(0x7ff8000000000000ULL);
                 }
-                reinterpret_cast<double2 *>(P.out + 4 * i)[0] = make_double2(s[0], s[1]);
-                reinterpret_cast<double2 *>(P.out + 4 * i)[1] = make_double2(s[2], s[3]);
+                if (aligned32) {
+                    store_32_bytes(P.out + 4 * i, s);
+                } else {
+                    reinterpret_cast<double2 *>(P.out + 4 * i)[0] = make_double2(s[0], s[1]);
+                    reinterpret_cast<double2 *>(P.out + 4 * i)[1] = make_double2(s[2], s[3]);
+                }
             }
         } else {
             if (ORDERED) W.place[lane].cell0 = (uint32_t)i;
