@@ -719,6 +719,20 @@ __device__ __forceinline__ Geo camera_geo(const ViewDev &v, const CameraRay &c) 
     return g;
 }
 
+// First slot of the queue's pack of 32 rays at `base`: the packs are taken from
+// the middle of the slots outwards.  A view's middle rows hold the rays that
+// pass the hole, with several times the steps of its edges; in slot order the
+// last warps to fetch a pack, with nothing left to share, were often among
+// them.  512 x 512 rays, learned 4.82 -> 3.88 ms, controller 3.21 -> 2.62; 400 x
+// 400 2.93 -> 2.64 and 2.14 -> 1.80; from 900 x 900 on, many packs per warp, even.
+// While every warp gets at most one pack the order shapes no tail, and only
+// parts neighbours (200 x 200: 2.19 against 2.41 ms): slot order there.
+__device__ __forceinline__ unsigned long long middle_out(unsigned long long base, unsigned long long total) {
+    const unsigned long long packs = (total + 31) >> 5, k = base >> 5, mid = packs >> 1;
+    if (packs <= (unsigned long long)gridDim.x * (blockDim.x >> 5)) return base;
+    return ((k & 1) ? mid - ((k + 1) >> 1) : mid + (k >> 1)) << 5;
+}
+
 // Step-doubling controller: renders the adaptive image and records samples.
 // DRIFT: track each ray's Hamiltonian drift (only when it is asked for).
 template <bool DRIFT>
@@ -738,7 +752,7 @@ __global__ void __launch_bounds__(256) adaptive_kernel(const LearnParams L) {
         if (lane == 0) base = atomicAdd(&P.q->next, 32ull);
         base = __shfl_sync(kFull, base, 0);
         if (base >= total) break;
-        const unsigned long long slot = base + lane;
+        const unsigned long long slot = middle_out(base, total) + lane;
         if (slot < total) {
             const int vi = P.n_views == 1 ? 0 : find_view(vbegin, P.n_views, (int64_t)slot);
             const ViewDev &v = P.views[vi];
@@ -840,7 +854,7 @@ __global__ void __launch_bounds__(128, 5) learned_kernel(const LearnParams L) {
         if (lane == 0) base = atomicAdd(&P.q->next, 32ull);
         base = __shfl_sync(kFull, base, 0);
         if (base >= total) break;
-        const unsigned long long slot = base + lane;
+        const unsigned long long slot = middle_out(base, total) + lane;
         bool alive = slot < total;
         int vi = 0;
         PixelRef px;
