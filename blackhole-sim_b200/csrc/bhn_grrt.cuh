@@ -175,7 +175,11 @@ __global__ void __launch_bounds__(128) grrt_init_kernel(const TraceParams P, dou
     }
 }
 
-__global__ void __launch_bounds__(128) grrt_trace_kernel(const TraceParams P) {
+// One warp a block: the rays' chains of dependent FP64 steps set its time, so
+// few warps go to as many SMs as there are (144 rays 10.17 -> 9.94 ms a call in
+// blocks of 128 and of 32, 800 rays 12.46 -> 12.23; from 2,000 rays on, even).
+constexpr int kTraceThreads = 32;
+__global__ void __launch_bounds__(kTraceThreads) grrt_trace_kernel(const TraceParams P) {
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     __shared__ AxisHints hints;  // the snapshot axes' first-guess parameters (the whole block)
     load_axis_hints(hints, P.rg, P.nr, P.tg, P.nt, P.pg, P.np);
@@ -463,6 +467,7 @@ extern "C" int bhn_grrt_render(const double *fields, const double *r_grid, int32
     BHN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     BHN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grrt_coef_kernel, 128, 0));
     const unsigned ray_blocks = (unsigned)((rays + 127) / 128);
+    const unsigned trace_blocks = (unsigned)((rays + kTraceThreads - 1) / kTraceThreads);
     const unsigned coef_blocks = (unsigned)std::min<int64_t>((rays * chunk + 3) / 4, (int64_t)sms * std::max(per_sm, 1));
     BHN_CUDA_TRY(cudaMemsetAsync(W.n_seg, 0, sizeof(unsigned long long), s));
     grrt_init_kernel<<<ray_blocks, 128, 0, s>>>(T, out, diag);
@@ -470,7 +475,7 @@ extern "C" int bhn_grrt_render(const double *fields, const double *r_grid, int32
     // every round either ends a ray's trace or lists chunk segments of it, one step each at least
     const int64_t rounds = (int64_t)cfg->max_steps / chunk + 2;
     for (int64_t k = 0; k < rounds; ++k) {
-        grrt_trace_kernel<<<ray_blocks, 128, 0, s>>>(T);
+        grrt_trace_kernel<<<trace_blocks, kTraceThreads, 0, s>>>(T);
         BHN_LAUNCH_CHECK("grrt_trace_kernel");
         grrt_coef_kernel<<<coef_blocks, 128, 0, s>>>(C);
         BHN_LAUNCH_CHECK("grrt_coef_kernel");
