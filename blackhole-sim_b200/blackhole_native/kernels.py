@@ -279,7 +279,9 @@ def _launch_sample_and_step(c, rg, tg, pg, pts, n: int, ds: float, ini, policy: 
     L = _lib.lib()
     args = (dev.ptr(c), dev.ptr(rg), rg.numel(), dev.ptr(tg), tg.numel(), dev.ptr(pg), pg.numel(), dev.ptr(pts), n, ds,
             dev.ptr(ini), ini.numel(), policy, dev.ptr(out))
-    scratch, sp, nbytes = _sort_scratch(n, rg.numel() * tg.numel() * pg.numel(), out.device)
+    scratch = None
+    if n >= SORT_MIN_POINTS:
+        scratch, sp, nbytes = _sort_scratch(n, rg.numel() * tg.numel() * pg.numel(), out.device)
     if scratch is None:
         _lib.check(L.bhn_sample_and_step_stokes(*args, dev.stream_ptr()))
         return
@@ -291,7 +293,9 @@ def _launch_sample_trilinear(c, rg, tg, pg, pts, n: int, out) -> None:
     L = _lib.lib()
     args = (dev.ptr(c), dev.ptr(rg), rg.numel(), dev.ptr(tg), tg.numel(), dev.ptr(pg), pg.numel(), dev.ptr(pts), n,
             dev.ptr(out))
-    scratch, sp, nbytes = _sort_scratch(n, rg.numel() * tg.numel() * pg.numel(), out.device)
+    scratch = None
+    if n >= SORT_MIN_POINTS:
+        scratch, sp, nbytes = _sort_scratch(n, rg.numel() * tg.numel() * pg.numel(), out.device)
     if scratch is None:
         _lib.check(L.bhn_sample_brick_trilinear(*args, dev.stream_ptr()))
         return

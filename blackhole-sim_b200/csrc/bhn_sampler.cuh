@@ -23,6 +23,7 @@ constexpr int kGridSmem = 4096;  // knots of the three axes kept in shared memor
 struct SamplePoints {
     const double *coeffs, *rg, *tg, *pg, *pts, *initial;
     int nr, nt, np, broadcast, policy;
+    int per_warp;                  // input order: points a warp takes at a time (32 in cell order)
     int64_t n;
     double ds;
     double *out;
@@ -151,14 +152,15 @@ __global__ void __launch_bounds__(kSampleThreads, kSampleBlocks) sample_points_k
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t ct = (uint32_t)P.np, cr = (uint32_t)(P.np * P.nt);  // cells to the next theta, r
     uint32_t bad = 0;
-    const int64_t step = (int64_t)gridDim.x * blockDim.x;
-    int64_t base = (int64_t)blockIdx.x * blockDim.x + 32 * warp;
+    const int group = ORDERED ? 32 : P.per_warp;
+    const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5) * group;
+    int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + warp) * group;
     uint32_t next_i = 0, next_key = P.invalid_key;
     double nr_ = 0.0, nt_ = 0.0, np_ = 0.0;
     const bool aligned16 = (reinterpret_cast<uintptr_t>(P.pts) & 15) == 0;  // else three 8-byte reads
     const bool aligned32 = (reinterpret_cast<uintptr_t>(P.out) & 31) == 0;  // else two 16-byte writes
     auto fetch = [&](int64_t k) {  // point k of the order (k < n) into next_*
-        if (k >= P.n) return;
+        if (k >= P.n || (!ORDERED && lane >= group)) return;
         int64_t i = k;
         if (ORDERED) {
             next_i = __ldcs(P.order + k);
@@ -186,7 +188,8 @@ __global__ void __launch_bounds__(kSampleThreads, kSampleBlocks) sample_points_k
         bool inside = false;
         int r0 = 0, t0 = 0, p0 = 0;
         double wr = 0.0, wt = 0.0, wp = 0.0;
-        if (k < P.n) {
+        const bool mine = k < P.n && (ORDERED || lane < group);
+        if (mine) {
             const double p = wrap_phi(ph, A.p[0]);
             if (ORDERED) {
                 inside = next_key != P.invalid_key;
@@ -217,7 +220,7 @@ __global__ void __launch_bounds__(kSampleThreads, kSampleBlocks) sample_points_k
         fetch(k + step);
         __syncwarp();
 #pragma unroll kCornerUnroll
-        for (int j = 0; j < 11; ++j) {
+        for (int j = 0; j < (ORDERED ? 11 : (11 * group + 31) >> 5); ++j) {
             const int item = lane + 32 * j, pt = item / 11, ch = item - 11 * pt;
             if (in_mask >> pt & 1) {
                 const Place w = W.place[pt];
@@ -239,7 +242,7 @@ __global__ void __launch_bounds__(kSampleThreads, kSampleBlocks) sample_points_k
         }
         __syncwarp();
         if (STEP) {
-            if (k < P.n) {
+            if (mine) {
                 const double *s0 = P.initial + (P.broadcast ? 0 : 4 * i);
                 double s[4] = {s0[0], s0[1], s0[2], s0[3]};
                 if (inside) {
@@ -263,10 +266,10 @@ __global__ void __launch_bounds__(kSampleThreads, kSampleBlocks) sample_points_k
             if (ORDERED) W.place[lane].cell0 = (uint32_t)i;
             __syncwarp();
 #pragma unroll 1
-            for (int j = 0; j < 11; ++j) {
+            for (int j = 0; j < (ORDERED ? 11 : (11 * group + 31) >> 5); ++j) {
                 const int item = lane + 32 * j, pt = item / 11;
                 const int64_t o = ORDERED ? (int64_t)W.place[pt].cell0 : base + pt;
-                if (base + pt < P.n) P.out[11 * o + item - 11 * pt] = W.value[item];
+                if (base + pt < P.n && (ORDERED || pt < group)) P.out[11 * o + item - 11 * pt] = W.value[item];
             }
         }
         __syncwarp();

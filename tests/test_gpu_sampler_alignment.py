@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 import torch
 
+import blackhole_native as bn
 from blackhole_native import _device as dev, _lib
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +41,20 @@ def test_alignments_agree(n, pts_offset, out_offset):
         assert bool((out[:out_offset] == 7.0).all()) and bool((out[out_offset + 4 * n:] == 7.0).all())
         got.append(out[out_offset:out_offset + 4 * n].view(torch.int64).clone())
     assert torch.equal(*got)
+
+
+@pytest.mark.parametrize("per_warp", [4, 8, 16])
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+def test_points_per_warp(per_warp, extra):
+    """Around the point counts where a warp's share changes: a call equals its points in calls of other shares."""
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 32 * per_warp + extra
+    rng = np.random.default_rng(n)
+    nr, nt, npz = 9, 7, 6
+    axes = [torch.as_tensor(g, device="cuda") for g in
+            (np.linspace(1.0, 9.0, nr), np.linspace(0.2, 2.9, nt), np.linspace(0.0, 5.9, npz))]
+    c = torch.as_tensor(rng.normal(size=nr * nt * npz * 11), device="cuda")
+    pts = torch.as_tensor(rng.uniform([0.8, 0.1, -9.0], [9.2, 3.0, 9.0], (n, 3)).ravel(), device="cuda")
+    whole = bn.sample_brick_trilinear(c, *axes, pts)
+    cuts = [0, 7, n // 5, n // 2, n]
+    parts = torch.cat([bn.sample_brick_trilinear(c, *axes, pts[3 * a:3 * b]) for a, b in zip(cuts, cuts[1:])])
+    assert torch.equal(whole.view(torch.int64), parts.view(torch.int64))
