@@ -1201,7 +1201,7 @@ def bench_micro(args) -> dict | None:
     peaks = load_peaks()
     stokes_rk2 = {"cells_per_step": cells, "ms_per_step": rk_ms, "cells_per_s": cells / (rk_ms * 1e-3),
                   "roofline": {"bound": "hbm", "achieved": round(rk_gbs, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                               "frac": round(rk_gbs / peaks["hbm_gbs"], 4), "kernel": "stokes_rk2_brick_kernel",
+                               "frac": round(rk_gbs / peaks["hbm_gbs"], 4), "kernel": "stokes_brick_kernel<false>",
                                "algorithmic_bytes_per_cell": 120}}
 
     cpu = None
@@ -1224,7 +1224,7 @@ def bench_micro(args) -> dict | None:
                      "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": profiled_traffic(MICRO_PROFILE),
                      "peak_source": f"{peaks['source']} (MEASURED_PEAKS.json hbm_gbs)" if peaks["source"] == "measured"
                      else "fallback 6.65 TB/s",
-                     "kernel": "sample_and_step_ordered_kernel (timed: cell keys, radix sort and the ordered "
+                     "kernel": "sample_points_kernel<true, true> (timed: cell keys, radix sort and the ordered "
                                "sampler)", "algorithmic_bytes_per_point": MICRO_BYTES_PER_POINT},
         "cpu_baseline": cpu,
         "kernel_ms": {"mean": per_mean, "min": min(per), "max": max(per)},

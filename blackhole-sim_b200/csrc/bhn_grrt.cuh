@@ -13,8 +13,8 @@
 // step, until tau reaches the cutoff.
 //
 // Wavefront form.  The geodesic is a long chain of dependent FP64 steps per
-// ray and the coefficients are ~10^4 independent exp() evaluations per
-// emitting segment, so they run as separate kernels, in rounds:
+// ray and the coefficients are ~1,500 independent instructions per emitting
+// segment, so they run as separate kernels, in rounds:
 //   trace_kernel     one thread per ray: continues its RK4 geodesic until it
 //                    has produced `chunk` emitting segments (or the trace
 //                    ends), appending each segment's plasma frame to a list;
