@@ -30,8 +30,9 @@ static int frames_per_warp(int64_t n, int sms) {
 
 // Six 128-thread blocks per SM (80 registers): 30,011 Hybrid frames took 188
 // us against 242 at five and 193 at seven and eight, before the power law's
-// nodes were grouped.  Now 100 us and 35 us for the tables (728 us with one
-// frame per warp and two exp() per node and pitch angle), 2.5 ns a frame at a
+// nodes were grouped.  Now 93 us and 27 us for the tables (728 us with one
+// frame per warp and two exp() per node and pitch angle; 100 and 35 while the
+// blocks copied their tables through the constant bank), 2.5 ns a frame at a
 // million and more (22.6).  Leaving out the row lookups takes three quarters
 // of it, cheap stand-ins for log or exp 9 % each; the issue slots are two
 // thirds busy, fixed FP64 latencies and the shared-memory round trip of
@@ -205,9 +206,10 @@ struct TableParams {
 // then one of the two kernels' coefficients; the last block makes the power
 // law's nodes.  Tens of thousands of rows and no reuse: bound by the FP64 work
 // of a term (two exponentials, 24 moments) and a row (economisation).  The
-// default Hybrid model's 39,892 rows take 35 us (four lanes 43, with two more
-// rounds of 24 shuffles); 51 us with a product more per moment and with the
-// rows past the far tail, a fifth of them, which no lookup reaches.
+// default Hybrid model's 39,892 rows take 27 us (35 with the knots copied
+// through the constant bank, then 43 with four lanes a row and two more rounds
+// of 24 shuffles); 51 us with a product more per moment and with the rows past
+// the far tail, a fifth of them, which no lookup reaches.
 constexpr int kRowLanes = 2;
 __global__ void __launch_bounds__(128) sum_table_kernel(const __grid_constant__ TableParams P) {
     __shared__ KernelTable K;
@@ -241,12 +243,13 @@ __global__ void __launch_bounds__(128) sum_table_kernel(const __grid_constant__ 
         if (threadIdx.x == 0) *P.nt_norm = (part[0] + part[1]) + (part[2] + part[3]);
         return;
     }
+    const KernelTable &source = *lane_reads(&P.K);
     for (int i = threadIdx.x; i < kTable; i += blockDim.x) {
-        K.lx[i] = P.K.lx[i];
-        K.lF[i] = P.K.lF[i];
-        K.lG[i] = P.K.lG[i];
-        K.sF[i] = P.K.sF[i];
-        K.sG[i] = P.K.sG[i];
+        K.lx[i] = source.lx[i];
+        K.lF[i] = source.lF[i];
+        K.lG[i] = source.lG[i];
+        K.sF[i] = source.sF[i];
+        K.sG[i] = source.sG[i];
     }
     __syncthreads();
     const int part = threadIdx.x % kRowLanes;

@@ -215,7 +215,8 @@ struct Integrals {
 // coefficients of its two degrees by the node's w z^degree from shared memory,
 // and the sum over the degrees falls to the reduction that sums the nodes:
 // 13.7 ms with eight lanes and 16 bytes.  The wide loads and paired powers
-// halve the exchange's instructions: 30,011 Hybrid frames 106.6 -> 100.1 us.
+// halve the exchange's instructions: 30,011 Hybrid frames 106.6 -> 100.1 us (92.9
+// with lane_reads).
 // A node whose smallest x (the pitch with the largest sin) already lies in
 // the table's far tail adds terms below kTailValue times the pitch weights
 // (< 1e-270): nothing a cell that emits can resolve.  Skipping it leaves such
@@ -375,8 +376,19 @@ __device__ __forceinline__ void add_rotated(double *out, double jI, double jQ, d
 }
 
 
+// A pointer to a kernel parameter for reads that differ from lane to lane: plain
+// loads through its generic address.  Left to the parameters' constant bank, a
+// warp's read of 32 addresses is 32 reads: every block's copy of its tables took
+// about 7 us (30,011 frames 99.5 -> 92.9 us, their tables 34.9 -> 26.7).
+template <typename T>
+__device__ __forceinline__ const T *lane_reads(const T *p) {
+    asm volatile("" : "+l"(p));
+    return p;
+}
+
 // Block-cooperative copy of the interval searches into shared memory.
-__device__ __forceinline__ void load_pieces(PieceSmem &S, const SumTable &T) {
+__device__ __forceinline__ void load_pieces(PieceSmem &S, const SumTable &table) {
+    const SumTable &T = *lane_reads(&table);
     for (int i = threadIdx.x; i < kMaxCells; i += blockDim.x) {
         S.cell[i] = T.cell[i];
         if (i <= kMaxPieces) S.edge[i] = i < T.pieces ? T.edge[i] : INFINITY;
