@@ -469,8 +469,10 @@ void set_table(SumTable &T, const SumPlan &P, const double2 *rows) {
 
 // Power-law nodes per row: 8 (28 rows of the default 224 nodes, one per lane)
 // while the group's sum has at most 64 terms and its span fits the cells, once
-// the frames repay its table.
-constexpr int64_t kGroupFrames = 16384;
+// the frames repay its table (a call without and with groups: 5,000 Hybrid frames
+// 53.6 and 59.6 us, 8,192 67.5 and 65.8; power law alone 4,000 38.6 and 41.2,
+// 8,192 47.5 and 43.5, 12,000 60.6 and 47.3).
+constexpr int64_t kGroupFrames = 8192;
 int group_size(const SumPlan &A, int gamma_n, double lr, int64_t frames) {
     int g = 1;
     while (frames >= kGroupFrames && 2 * g * A.n <= 64 && 2 * g <= 8 && 2 * g <= gamma_n &&

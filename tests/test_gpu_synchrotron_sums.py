@@ -16,7 +16,7 @@ import blackhole_native as bn
 from oracle import synchrotron as S
 
 pytestmark = pytest.mark.gpu
-GROUPED = 16384  # frames from which the power law's nodes are taken in groups
+GROUPED = 8192  # frames from which the power law's nodes are taken in groups
 
 
 def _frames(n, seed):
