@@ -530,7 +530,10 @@ int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, void *
         make_plan(T.plan[0]);
         rows[0] = T.plan[0].rows;
     }
-    if (M.nt.on) {
+    // A power law without an upper end has no grid of nodes (its log ratio is infinite, and so would the group's
+    // shifts be): every integral over it is indefinite, which the coefficients report as no emission.
+    const bool nt_nodes = M.nt.on && std::isfinite(M.nt.gamma_max);
+    if (nt_nodes) {
         pitch_terms(m->nonthermal_pitch_n, T.plan[2]);
         make_plan(T.plan[2]);
         const SumPlan &A = T.plan[2];
@@ -567,8 +570,10 @@ int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, void *
         if (rows[k]) T.rows[k] = next;
         next += 8 * rows[k];
     }
-    if (M.nt.on) T.nt_nodes = next;
-    T.nt_norm = reinterpret_cast<double *>(next + M.nt_groups + M.nt_single);
+    if (nt_nodes) {
+        T.nt_nodes = next;
+        T.nt_norm = reinterpret_cast<double *>(next + M.nt_groups + M.nt_single);
+    }
     const unsigned blocks = (unsigned)((kRowLanes * total + 127) / 128 + 1);
     sum_table_kernel<<<blocks, 128, 0, stream>>>(T);
     if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) {
@@ -577,7 +582,7 @@ int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, void *
         return cuda_fail(e, "sum_table_kernel");
     }
     if (M.th.on) set_table(M.tth, T.plan[0], T.rows[0]);
-    if (M.nt.on) {
+    if (nt_nodes) {
         set_table(M.tnt, T.plan[1], T.rows[same[1]]);
         set_table(M.tnt1, T.plan[2], T.rows[same[2]]);
     }

@@ -120,7 +120,7 @@ struct Model {
     SumTable tnt, tnt1;       // power law: a group of nodes; the pitch average (its ungrouped nodes)
     int nt_groups, nt_single;
     const double2 *nt_nodes;  // power law: (weight, 2 log gamma) of every group, then of the ungrouped nodes
-    const double *nt_norm;    // the sum of all nodes' weights
+    const double *nt_norm;    // the sum of all nodes' weights (NULL: a power law without an upper end, no nodes)
 };
 
 // Shared-memory copy of a table's interval search.
@@ -452,7 +452,7 @@ __device__ __forceinline__ void coefficients(TableSmem &S, const Model &M, const
             if (lane == src) nt = r;
         }
         if (emits) powerlaw_single(M, S.nt1, base, nt);
-        nt.norm = __ldg(M.nt_norm);
+        nt.norm = M.nt_norm ? __ldg(M.nt_norm) : 0.0;
     }
     if (!emits) return;
     const double n_e = f.n_e, te = f.te, b = f.b, nu = f.nu;
