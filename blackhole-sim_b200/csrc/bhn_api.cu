@@ -411,8 +411,7 @@ int launch_samples(SamplePoints P, bool step, cudaStream_t s) {
     const int64_t blocks = std::min(resident, (32 * groups + threads - 1) / threads);
     const int smem = (int)sizeof(WarpPoints) * (threads / 32) + grid_smem(P.nr, P.nt, P.np);
     auto go = [&](auto kernel) -> int {
-        if (smem > 48 * 1024)
-            BHN_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        if (int rc = smem > 48 * 1024 ? allow_dynamic_smem(kernel, kSampleSmem) : 0) return rc;
         kernel<<<(unsigned)blocks, threads, smem, s>>>(P);
         BHN_LAUNCH_CHECK("sample_points_kernel");
         return BHN_OK;

@@ -21,6 +21,16 @@ int sm_count_current_device();
 int stream_alloc(void **p, int64_t bytes, cudaStream_t s);
 void stream_free(void *p, cudaStream_t s);
 
+// Lets launches of `kernel` ask for up to `most` bytes of dynamic shared memory.
+// The limit belongs to the function, not to a launch, so it is the same constant
+// in every call: a limit set to one call's own size could be lowered by another
+// host thread between that call's setting and its launch, which then fails.
+template <class Kernel>
+int allow_dynamic_smem(Kernel kernel, int most) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    return e == cudaSuccess ? 0 : cuda_fail(e, "cudaFuncSetAttribute");
+}
+
 #define BHN_CUDA_TRY(expr)                                   \
     do {                                                     \
         cudaError_t e_ = (expr);                             \

@@ -1011,7 +1011,7 @@ static int learn_params(const void *records, const void *tables, int32_t nr, int
     if (scratch_bytes < SL.total) return fail(BHN_ERR_VALUE, "scratch buffer is smaller than bhn_render_scratch_bytes()");
     const int tables_bytes = (int)table_layout(nr, nt, np).total;
     const int64_t sm = smem_bytes(tables_bytes, n_views);
-    if (sm > 160 * 1024) return fail(BHN_ERR_VALUE, "brick grids plus views exceed the shared-memory table budget");
+    if (sm > kLearnSmem) return fail(BHN_ERR_VALUE, "brick grids plus views exceed the shared-memory table budget");
     smem = (int)sm;
     char *sc = static_cast<char *>(scratch);
     memset(&L, 0, sizeof L);
@@ -1078,7 +1078,7 @@ int bhn_mlp_grad(const float *params, const float *samples, const int64_t *index
                  float *grad, float *loss, void *stream) {
     if (count < 1) return fail(BHN_ERR_VALUE, "batch must contain at least one sample");
     const int smem = (int)sizeof(TrainSmem);
-    BHN_CUDA_TRY(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (int rc = allow_dynamic_smem(mlp_grad_kernel, smem)) return rc;
     const unsigned blocks = (unsigned)((count + kTrainBlock - 1) / kTrainBlock);
     mlp_grad_kernel<<<blocks, kTrainThreads, smem, as_stream(stream)>>>(
         params, samples, index, first, count, grad, loss, (reinterpret_cast<uintptr_t>(grad) & 15) == 0);
@@ -1137,8 +1137,7 @@ int bhn_adaptive_launch(const void *records, const void *tables, int32_t nr, int
     L.counters = counters;
     const int sms = sm_count_current_device();
     auto go = [&](auto kernel) -> int {
-        if (smem > 48 * 1024)
-            BHN_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        if (int rc = smem > 48 * 1024 ? allow_dynamic_smem(kernel, kLearnSmem) : 0) return rc;
         kernel<<<sms * cfg->blocks_per_sm, cfg->block_threads, smem, s>>>(L);
         BHN_LAUNCH_CHECK("adaptive_kernel");
         return BHN_OK;
@@ -1161,8 +1160,7 @@ int bhn_learned_launch(const void *records, const void *tables, int32_t nr, int3
     const int sms = sm_count_current_device();
     const unsigned blocks = sms * cfg->blocks_per_sm * (cfg->block_threads / 128 > 0 ? cfg->block_threads / 128 : 1);
     auto go = [&](auto kernel) -> int {
-        if (smem > 48 * 1024)
-            BHN_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        if (int rc = smem > 48 * 1024 ? allow_dynamic_smem(kernel, kLearnSmem) : 0) return rc;
         kernel<<<blocks, 128, smem, s>>>(L);
         BHN_LAUNCH_CHECK("learned_kernel");
         return BHN_OK;

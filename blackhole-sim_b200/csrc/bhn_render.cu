@@ -963,6 +963,8 @@ __host__ __device__ inline int64_t smem_bytes(int tables_bytes, int n_views) {
            align16(sizeof(BlockCounters)) + align16(8 * ((int64_t)n_views + 1));
 }
 
+constexpr int kRenderSmem = 200 * 1024, kLearnSmem = 160 * 1024;  // the most smem_bytes that a launch takes
+
 // ------------------------------------------------------------ persistent loop
 // MINB = resident 256-thread blocks the register allocation must allow:
 // 1 -> unconstrained, 3 -> <= 85 registers, 4 -> <= 64 registers.
@@ -1186,7 +1188,7 @@ static int launch_render(const void *records, const void *tables, int32_t nr, in
         return fail(BHN_ERR_VALUE, "records/tables/out must be 16-byte and scratch 256-byte aligned");
     const int tables_bytes = (int)table_layout(nr, nt, np).total;
     const int64_t smem64 = smem_bytes(tables_bytes, n_views);
-    if (smem64 > 200 * 1024) return fail(BHN_ERR_VALUE, "brick grids plus views exceed the shared-memory table budget");
+    if (smem64 > kRenderSmem) return fail(BHN_ERR_VALUE, "brick grids plus views exceed the shared-memory table budget");
     const int smem = (int)smem64;
     char *sc = static_cast<char *>(scratch);
     RenderParams P;
@@ -1215,8 +1217,7 @@ static int launch_render(const void *records, const void *tables, int32_t nr, in
     BHN_CUDA_TRY(cudaMemsetAsync(&P.q->next, 0, sizeof(unsigned long long), s));
     BHN_CUDA_TRY(cudaMemsetAsync(P.stats, 0, sizeof(bhn_render_stats), s));
     auto go = [&](auto kernel) -> int {
-        if (smem > 48 * 1024)
-            BHN_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        if (int rc = smem > 48 * 1024 ? allow_dynamic_smem(kernel, kRenderSmem) : 0) return rc;
         kernel<<<grid, block, smem, s>>>(P);
         BHN_LAUNCH_CHECK("render_kernel");
         return BHN_OK;

@@ -138,6 +138,7 @@ struct WarpPoints {
     Place place[32];
     double value[32 * 11];
 };
+constexpr int kSampleSmem = (int)sizeof(WarpPoints) * (kSampleThreads / 32) + 8 * kGridSmem;  // the most a launch takes
 // Four doubles in one 32-byte store (32-byte aligned).
 __device__ __forceinline__ void store_32_bytes(double *p, const double (&v)[4]) {
     asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]) : "memory");
