@@ -510,7 +510,7 @@ int order_points_by_cell(SamplePoints &P, const SortLayout &L, void *scratch, cu
     uint32_t *idx_sorted = reinterpret_cast<uint32_t *>(base + L.idx_out);
     const uint32_t cells = (uint32_t)((int64_t)P.nr * P.nt * P.np);
     AxisHints *hints = reinterpret_cast<AxisHints *>(base + L.hints);
-    axis_hints_kernel<<<1, 32, 0, s>>>(P.rg, P.nr, P.tg, P.nt, P.pg, P.np, hints);
+    axis_hints_kernel<<<3, kHintThreads, 0, s>>>(P.rg, P.nr, P.tg, P.nt, P.pg, P.np, hints);
     BHN_LAUNCH_CHECK("axis_hints_kernel");
     cell_key_kernel<<<grid_for(P.n, 256), 256, grid_smem(P.nr, P.nt, P.np), s>>>(
         P.rg, P.nr, P.tg, P.nt, P.pg, P.np, P.pts, P.n, cells, hints, keys_in, idx_in, P.bad_points);
