@@ -188,7 +188,7 @@ __global__ void build_tables_kernel(const double *__restrict__ rg, int nr, const
             kind = kUniform;
             inv = 1.0 / d;
             off = g[0] * inv;
-        } else if (g[0] > 0.0) {
+        } else if (threadIdx.x < 2 && g[0] > 0.0) {  // locate_phi_f and locate_phi know no geometric guess
             double dl = log(g[n - 1] / g[0]) / (n - 1);
             double devl = 0.0;
             for (int i = 0; i < n; ++i) devl = fmax(devl, fabs(log(g[i] / g[0]) - i * dl));

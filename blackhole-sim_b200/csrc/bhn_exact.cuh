@@ -57,7 +57,7 @@ __device__ __forceinline__ bool lerp_cells(const double *__restrict__ coeffs, in
 // First-guess parameters of the three brick axes (r, theta, phi), classified
 // once per block by its first warp: uniform when every knot lies within a
 // quarter cell of g0 + k d, geometric when within a quarter cell of
-// g0 exp(k dl), else binary search (the rule of build_tables_kernel).
+// g0 exp(k dl) (r and theta), else binary search (the rule of build_tables_kernel).
 struct AxisHints {
     int kind[3];
     double off[3], inv[3];
@@ -92,7 +92,8 @@ __device__ __forceinline__ void classify_axis(const double *g, int n, int first,
 }
 __device__ __forceinline__ void set_axis_hint(AxisHints &h, int a, const double *g, int n, int kind, double off,
                                               double inv) {
-    h.kind[a] = isfinite(off) && isfinite(inv) ? kind : kSearch;
+    if (!(isfinite(off) && isfinite(inv)) || (a == 2 && kind == kGeometric)) kind = kSearch;  // phi's guess is the uniform one
+    h.kind[a] = kind;
     h.off[a] = off;
     h.inv[a] = inv;
     h.g0[a] = g[0];
