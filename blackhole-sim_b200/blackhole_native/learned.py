@@ -320,7 +320,9 @@ def count_samples(brick: DeviceBrick, views: Sequence[View], adapt: AdaptConfig)
 
 
 def generate_samples(brick: DeviceBrick, views: Sequence[View], adapt: AdaptConfig, capacity: int) -> torch.Tensor:
-    """Run the controller and return the recorded (features, log multiplier) rows."""
+    """Run the controller and return the recorded (features, log multiplier)
+    rows.  More rows than ``capacity`` (``count_samples`` tells how many there
+    are): the ones recorded first are kept, of the views' first rays."""
     samples = torch.empty((capacity, 9), dtype=torch.float32, device=brick.device)
     count = torch.zeros(1, dtype=torch.int64, device=brick.device)
     render_adaptive(brick, views, adapt, samples=samples, sample_count=count)

@@ -734,6 +734,8 @@ __device__ __forceinline__ unsigned long long middle_out(unsigned long long base
 }
 
 // Step-doubling controller: renders the adaptive image and records samples.
+// Recording launches take the rays in slot order: a buffer that fills up keeps
+// the rows that come first, and those are the image's first rays.
 // DRIFT: track each ray's Hamiltonian drift (only when it is asked for).
 template <bool DRIFT>
 __global__ void __launch_bounds__(256) adaptive_kernel(const LearnParams L) {
@@ -752,7 +754,7 @@ __global__ void __launch_bounds__(256) adaptive_kernel(const LearnParams L) {
         if (lane == 0) base = atomicAdd(&P.q->next, 32ull);
         base = __shfl_sync(kFull, base, 0);
         if (base >= total) break;
-        const unsigned long long slot = middle_out(base, total) + lane;
+        const unsigned long long slot = (L.samples ? base : middle_out(base, total)) + lane;
         if (slot < total) {
             const int vi = P.n_views == 1 ? 0 : find_view(vbegin, P.n_views, (int64_t)slot);
             const ViewDev &v = P.views[vi];
