@@ -26,7 +26,7 @@ import torch
 
 from . import _device as dev
 from . import _lib
-from .synchrotron import HybridSynchrotronCoefficients, ModelStruct, model_struct
+from .synchrotron import HybridSynchrotronCoefficients, ModelStruct, model_struct, table_scratch
 
 G_CGS = 6.67430e-8       # calibration.py:19
 C_CGS = 2.99792458e10    # calibration.py:18
@@ -160,11 +160,11 @@ def _declare() -> ctypes.CDLL:
     L = _lib.lib()
     L.bhn_grrt_scratch_bytes.argtypes = [ctypes.c_int64, ctypes.c_int32]
     L.bhn_grrt_scratch_bytes.restype = ctypes.c_int64
-    fn = L.bhn_grrt_render
-    vp, i32 = ctypes.c_void_p, ctypes.c_int32
-    fn.argtypes = [vp, vp, i32, vp, i32, vp, i32, ctypes.POINTER(_lib.ViewStruct), ctypes.POINTER(ModelStruct),
-                   ctypes.POINTER(GrrtConfigStruct), vp, ctypes.c_int64, vp, vp, vp]
-    fn.restype = ctypes.c_int
+    vp, i32, i64 = ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64
+    for fn, tables in ((L.bhn_grrt_render, []), (L.bhn_grrt_render_scratch, [vp, i64])):
+        fn.argtypes = [vp, vp, i32, vp, i32, vp, i32, ctypes.POINTER(_lib.ViewStruct), ctypes.POINTER(ModelStruct),
+                       ctypes.POINTER(GrrtConfigStruct), vp, i64, *tables, vp, vp, vp]
+        fn.restype = ctypes.c_int
     return L
 
 
@@ -265,9 +265,11 @@ def render_stokes_image_device(cfg, snapshot, scaling, *, coeff_model=None, diag
         raise ValueError("out must be a contiguous (H, W, 4) float64 tensor on the snapshot's device")
     diag = torch.empty((v.height, v.width, 8), dtype=torch.float64, device=device) if diagnostics else None
     g = ds.grids
-    _lib.check(L.bhn_grrt_render(dev.ptr(ds.fields), dev.ptr(g[0]), g[0].numel(), dev.ptr(g[1]), g[1].numel(),
-                                 dev.ptr(g[2]), g[2].numel(), ctypes.byref(v), ctypes.byref(m), ctypes.byref(c), sp,
-                                 nbytes, dev.ptr(out), dev.ptr(diag), dev.stream_ptr()))
+    tables = table_scratch(m, device)
+    _lib.check(L.bhn_grrt_render_scratch(dev.ptr(ds.fields), dev.ptr(g[0]), g[0].numel(), dev.ptr(g[1]), g[1].numel(),
+                                         dev.ptr(g[2]), g[2].numel(), ctypes.byref(v), ctypes.byref(m), ctypes.byref(c),
+                                         sp, nbytes, dev.ptr(tables), tables.numel(), dev.ptr(out), dev.ptr(diag),
+                                         dev.stream_ptr()))
     return (out, diag) if diagnostics else out
 
 

@@ -18,6 +18,8 @@ included.
 from __future__ import annotations
 
 import ctypes
+import functools
+import operator
 from dataclasses import dataclass, field
 from typing import Literal
 
@@ -126,8 +128,10 @@ class _DeviceCoefficients:
             raise ValueError("at least one plasma frame is required")
         out = torch.empty((n, 11), dtype=torch.float64, device=fd.device)
         m = model_struct(self, nu_hz, _UNIT_SCALING)
-        _lib.check(_declare_frames().bhn_synchrotron_coefficients(dev.ptr(fd), n, ctypes.byref(m), dev.ptr(out),
-                                                                  dev.stream_ptr()))
+        scratch = table_scratch(m, fd.device)
+        _lib.check(_declare_frames().bhn_synchrotron_coefficients_scratch(dev.ptr(fd), n, ctypes.byref(m), dev.ptr(out),
+                                                                          dev.ptr(scratch), scratch.numel(),
+                                                                          dev.stream_ptr()))
         return out if on_device else out.cpu().numpy()
 
     def coefficients(self, frame, nu_hz: float) -> PolarizedCoefficients:
@@ -203,22 +207,45 @@ class ModelStruct(ctypes.Structure):
     ]
 
 
+@functools.cache
 def _declare() -> ctypes.CDLL:
     L = _lib.lib()
-    fn = L.bhn_brick_precompute
-    vp = ctypes.c_void_p
-    fn.argtypes = [vp, vp, vp, ctypes.c_int64, ctypes.POINTER(ModelStruct), vp, ctypes.c_int32, vp]
-    fn.restype = ctypes.c_int
+    vp, i64, mp = ctypes.c_void_p, ctypes.c_int64, ctypes.POINTER(ModelStruct)
+    for fn, scratch in ((L.bhn_brick_precompute, []), (L.bhn_brick_precompute_scratch, [vp, i64])):
+        fn.argtypes = [vp, vp, vp, i64, mp, vp, ctypes.c_int32, *scratch, vp]
+        fn.restype = ctypes.c_int
     return L
 
 
+@functools.cache
 def _declare_frames() -> ctypes.CDLL:
     L = _lib.lib()
-    fn = L.bhn_synchrotron_coefficients
-    vp = ctypes.c_void_p
-    fn.argtypes = [vp, ctypes.c_int64, ctypes.POINTER(ModelStruct), vp, vp]
-    fn.restype = ctypes.c_int
+    vp, i64, mp = ctypes.c_void_p, ctypes.c_int64, ctypes.POINTER(ModelStruct)
+    for fn, scratch in ((L.bhn_synchrotron_coefficients, []), (L.bhn_synchrotron_coefficients_scratch, [vp, i64])):
+        fn.argtypes = [vp, i64, mp, vp, *scratch, vp]
+        fn.restype = ctypes.c_int
     return L
+
+
+TABLE_FIELDS = ("thermal", "nonthermal", "thermal_gamma_n", "thermal_pitch_n", "nonthermal_gamma_n",
+                "nonthermal_pitch_n", "nonthermal_gamma_min", "nonthermal_gamma_max")
+
+
+_table_values = operator.attrgetter(*TABLE_FIELDS)
+
+
+@functools.lru_cache(maxsize=64)
+def _table_bytes(values: tuple) -> int:
+    fn = _lib.lib().bhn_synchrotron_scratch_bytes
+    fn.argtypes, fn.restype = [ctypes.POINTER(ModelStruct)], ctypes.c_int64
+    return int(fn(ctypes.byref(ModelStruct(**dict(zip(TABLE_FIELDS, values))))))
+
+
+def table_scratch(m: ModelStruct, device) -> torch.Tensor:
+    """torch's memory for the model's tables of one call (for a model that the
+    library refuses, a stub: the call itself reports the error)."""
+    nbytes = _table_bytes(_table_values(m))
+    return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
 
 
 def model_struct(model, nu_hz: float, scaling) -> ModelStruct:
@@ -287,8 +314,10 @@ def precompute_device_coefficients(snapshot, scaling, nu_hz: float = 230e9,
     tdt = torch.float32 if dtype == "float32" else torch.float64
     out = torch.empty(shape + (11,), dtype=tdt, device=device)
     m = model_struct(coeff_model or HybridSynchrotronCoefficients(), nu_hz, scaling)
-    _lib.check(L.bhn_brick_precompute(dev.ptr(d_rho), dev.ptr(d_te), dev.ptr(d_b), cells, ctypes.byref(m),
-                                      dev.ptr(out), 4 if dtype == "float32" else 8, dev.stream_ptr()))
+    scratch = table_scratch(m, device)
+    _lib.check(L.bhn_brick_precompute_scratch(dev.ptr(d_rho), dev.ptr(d_te), dev.ptr(d_b), cells, ctypes.byref(m),
+                                              dev.ptr(out), 4 if dtype == "float32" else 8, dev.ptr(scratch),
+                                              scratch.numel(), dev.stream_ptr()))
     return r, theta, phi, out
 
 
@@ -356,6 +385,7 @@ def _precompute_pipelined(rho: np.ndarray, theta_e: np.ndarray, b_con: np.ndarra
              torch.empty(cap * 4, device=device, **f64)] for _ in range(2)]
     h_out = [torch.empty(cap * 11, dtype=tdt, **pinned) for _ in range(2)]
     d_out = [torch.empty(cap * 11, dtype=tdt, device=device) for _ in range(2)]
+    scratch = table_scratch(m, device)  # the slabs' kernels follow one another on one stream
     compute = torch.cuda.current_stream(device)
     up, down = torch.cuda.Stream(device), torch.cuda.Stream(device)
     up.wait_stream(compute)
@@ -386,9 +416,9 @@ def _precompute_pipelined(rho: np.ndarray, theta_e: np.ndarray, b_con: np.ndarra
         compute.wait_event(uploaded[j])
         if k >= 2:
             compute.wait_event(downloaded[j])  # slab k - 2's coefficients have left this device buffer
-        _lib.check(L.bhn_brick_precompute(dev.ptr(d_in[j][0]), dev.ptr(d_in[j][1]), dev.ptr(d_in[j][2]), n,
-                                          ctypes.byref(m), dev.ptr(d_out[j]), 4 if dtype == "float32" else 8,
-                                          compute.cuda_stream))
+        _lib.check(L.bhn_brick_precompute_scratch(dev.ptr(d_in[j][0]), dev.ptr(d_in[j][1]), dev.ptr(d_in[j][2]), n,
+                                                  ctypes.byref(m), dev.ptr(d_out[j]), 4 if dtype == "float32" else 8,
+                                                  dev.ptr(scratch), scratch.numel(), compute.cuda_stream))
         computed[j].record(compute)
         if k >= 1:
             finish(k - 1)  # while slab k computes; frees h_out[(k - 1) % 2] for slab k + 1

@@ -379,10 +379,10 @@ extern "C" int64_t bhn_grrt_scratch_bytes(int64_t rays, int32_t chunk) {
     return bhn::grrt_layout(rays, chunk).total;
 }
 
-extern "C" int bhn_grrt_render(const double *fields, const double *r_grid, int32_t nr, const double *theta_grid,
-                               int32_t nt, const double *phi_grid, int32_t np, const bhn_view *view,
-                               const bhn_synchrotron_model *model, const bhn_grrt_config *cfg, void *scratch,
-                               int64_t scratch_bytes, double *out, double *diag, void *stream) {
+static int grrt_render(const double *fields, const double *r_grid, int32_t nr, const double *theta_grid, int32_t nt,
+                       const double *phi_grid, int32_t np, const bhn_view *view, const bhn_synchrotron_model *model,
+                       const bhn_grrt_config *cfg, void *scratch, int64_t scratch_bytes, void *model_scratch,
+                       int64_t model_scratch_bytes, double *out, double *diag, void *stream) {
     using namespace bhn;
     if (!fields || !r_grid || !theta_grid || !phi_grid || !view || !cfg || !out || !scratch)
         return fail(BHN_ERR_VALUE, "missing snapshot, view, config or output buffer");
@@ -410,15 +410,10 @@ extern "C" int bhn_grrt_render(const double *fields, const double *r_grid, int32
                                        std::to_string(grrt_layout(rays, 1).total) + " bytes");
     cudaStream_t s = as_stream(stream);
     CoefParams C;
-    void *tables = nullptr;
+    synch::Scratch tables(model_scratch, model_scratch_bytes);
     // (a ray lists about a thousand segments; the same tables for every chunk, so the image does not depend on it)
     int rc = synch::build_model(model, rays * 1000, C.M, tables, s);
     if (rc) return rc;
-    struct Free {  // the model's tables, after the last kernel below
-        void *p;
-        cudaStream_t s;
-        ~Free() { stream_free(p, s); }
-    } free_tables{tables, s};
     rc = bhn_render_prepare(view, 1, scratch, scratch_layout(1).total, stream);  // FP64 camera tables of the view
     if (rc) return rc;
     const GrrtLayout GL = grrt_layout(rays, chunk);
@@ -483,4 +478,22 @@ extern "C" int bhn_grrt_render(const double *fields, const double *r_grid, int32
         BHN_LAUNCH_CHECK("grrt_transfer_kernel");
     }
     return BHN_OK;
+}
+
+extern "C" int bhn_grrt_render(const double *fields, const double *r_grid, int32_t nr, const double *theta_grid,
+                               int32_t nt, const double *phi_grid, int32_t np, const bhn_view *view,
+                               const bhn_synchrotron_model *model, const bhn_grrt_config *cfg, void *scratch,
+                               int64_t scratch_bytes, double *out, double *diag, void *stream) {
+    return grrt_render(fields, r_grid, nr, theta_grid, nt, phi_grid, np, view, model, cfg, scratch, scratch_bytes,
+                       nullptr, 0, out, diag, stream);
+}
+
+extern "C" int bhn_grrt_render_scratch(const double *fields, const double *r_grid, int32_t nr, const double *theta_grid,
+                                       int32_t nt, const double *phi_grid, int32_t np, const bhn_view *view,
+                                       const bhn_synchrotron_model *model, const bhn_grrt_config *cfg, void *scratch,
+                                       int64_t scratch_bytes, void *model_scratch, int64_t model_scratch_bytes,
+                                       double *out, double *diag, void *stream) {
+    if (!model_scratch) return bhn::fail(BHN_ERR_VALUE, "model scratch must not be NULL");
+    return grrt_render(fields, r_grid, nr, theta_grid, nt, phi_grid, np, view, model, cfg, scratch, scratch_bytes,
+                       model_scratch, model_scratch_bytes, out, diag, stream);
 }

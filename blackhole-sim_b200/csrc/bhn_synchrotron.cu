@@ -481,10 +481,13 @@ int group_size(const SumPlan &A, int gamma_n, double lr, int64_t frames) {
     return g;
 }
 
-}  // namespace
-
-int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, void *&tables, cudaStream_t stream) {
-    tables = nullptr;
+// The table plans of a model (T, under the lock), the model without its tables'
+// addresses (M) and the tables' size.
+TableParams T;  // ~25 KB: kept off the host stack; filled and launched under the lock
+std::mutex T_lock;
+int64_t T_rows[3];  // rows of each sum's own table (0: off, or another sum's)
+int T_same[3];      // which table serves each sum
+int plan_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, int64_t &bytes) {
     if (!m) return fail(BHN_ERR_VALUE, "synchrotron model must not be NULL");
     if (!std::isfinite(m->nu_hz)) return fail(BHN_ERR_VALUE, "nu_hz must be finite");
     auto check_comp = [](int on, int gn, int pn) {
@@ -517,23 +520,22 @@ int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, void *
         M.nt.absorption_scale = m->nonthermal_absorption_scale;
         M.nt.faraday_scale = m->nonthermal_faraday_scale;
     }
+    bytes = 0;
     if (!M.th.on && !M.nt.on) return BHN_OK;
-    static TableParams T;  // ~25 KB: kept off the host stack; filled and launched under the lock
-    static std::mutex lock;
-    std::lock_guard<std::mutex> g(lock);
     std::memset(&T, 0, sizeof T);
     T.K = host_table();
-    int64_t rows[3] = {0, 0, 0}, total = 0;
-    int same[3] = {0, 1, 2};  // which table serves each sum
+    for (int k = 0; k < 3; ++k) {
+        T_rows[k] = 0;
+        T_same[k] = k;
+    }
     if (M.th.on) {
         pitch_terms(m->thermal_pitch_n, T.plan[0]);
         make_plan(T.plan[0]);
-        rows[0] = T.plan[0].rows;
+        T_rows[0] = T.plan[0].rows;
     }
     // A power law without an upper end has no grid of nodes (its log ratio is infinite, and so would the group's
     // shifts be): every integral over it is indefinite, which the coefficients report as no emission.
-    const bool nt_nodes = M.nt.on && std::isfinite(M.nt.gamma_max);
-    if (nt_nodes) {
+    if (M.nt.on && std::isfinite(M.nt.gamma_max)) {
         pitch_terms(m->nonthermal_pitch_n, T.plan[2]);
         make_plan(T.plan[2]);
         const SumPlan &A = T.plan[2];
@@ -546,10 +548,10 @@ int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, void *
         T.gamma_max = M.nt.gamma_max;
         M.nt_groups = T.nt_n / T.nt_group;
         M.nt_single = 2 + std::max(0, T.nt_n - M.nt_groups * T.nt_group - 1);
-        if (M.th.on && m->thermal_pitch_n == m->nonthermal_pitch_n) same[2] = 0;
-        else rows[2] = A.rows;
+        if (M.th.on && m->thermal_pitch_n == m->nonthermal_pitch_n) T_same[2] = 0;
+        else T_rows[2] = A.rows;
         if (T.nt_group == 1) {
-            same[1] = same[2];
+            T_same[1] = T_same[2];
             B = A;
         } else {
             for (int i = 0; i < T.nt_group; ++i)
@@ -559,51 +561,59 @@ int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, void *
                     ++B.n;
                 }
             make_plan(B);
-            rows[1] = B.rows;
+            T_rows[1] = B.rows;
         }
     }
-    for (int k = 0; k < 3; ++k) total += rows[k];
-    int rc = stream_alloc(&tables, 128 * total + 16 * (int64_t)(M.nt_groups + M.nt_single + 1), stream);
-    if (rc) return rc;
-    double2 *next = static_cast<double2 *>(tables);
-    for (int k = 0; k < 3; ++k) {
-        if (rows[k]) T.rows[k] = next;
-        next += 8 * rows[k];
+    bytes = 128 * (T_rows[0] + T_rows[1] + T_rows[2]) + 16 * (int64_t)(M.nt_groups + M.nt_single + 1);
+    return BHN_OK;
+}
+
+}  // namespace
+
+int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, Scratch &tables, cudaStream_t stream) {
+    std::lock_guard<std::mutex> g(T_lock);
+    int64_t bytes = 0;
+    int rc = plan_model(m, frames, M, bytes);
+    if (rc || bytes == 0) return rc;
+    if (!tables.p) {
+        rc = stream_alloc(&tables.p, bytes, stream);
+        if (rc) return rc;
+        tables.owned = true;
+        tables.stream = stream;
+    } else if (tables.bytes < bytes || reinterpret_cast<uintptr_t>(tables.p) % 256) {
+        return fail(BHN_ERR_VALUE, "model scratch needs bhn_synchrotron_scratch_bytes() bytes, 256-byte aligned");
     }
-    if (nt_nodes) {
+    double2 *next = static_cast<double2 *>(tables.p);
+    for (int k = 0; k < 3; ++k) {
+        if (T_rows[k]) T.rows[k] = next;
+        next += 8 * T_rows[k];
+    }
+    if (M.nt_single) {
         T.nt_nodes = next;
         T.nt_norm = reinterpret_cast<double *>(next + M.nt_groups + M.nt_single);
     }
-    const unsigned blocks = (unsigned)((kRowLanes * total + 127) / 128 + 1);
+    const unsigned blocks = (unsigned)((kRowLanes * (T_rows[0] + T_rows[1] + T_rows[2]) + 127) / 128 + 1);
     sum_table_kernel<<<blocks, 128, 0, stream>>>(T);
-    if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) {
-        stream_free(tables, stream);
-        tables = nullptr;
-        return cuda_fail(e, "sum_table_kernel");
-    }
+    BHN_LAUNCH_CHECK("sum_table_kernel");
     if (M.th.on) set_table(M.tth, T.plan[0], T.rows[0]);
-    if (nt_nodes) {
-        set_table(M.tnt, T.plan[1], T.rows[same[1]]);
-        set_table(M.tnt1, T.plan[2], T.rows[same[2]]);
+    if (M.nt_single) {
+        set_table(M.tnt, T.plan[1], T.rows[T_same[1]]);
+        set_table(M.tnt1, T.plan[2], T.rows[T_same[2]]);
     }
     M.nt_nodes = T.nt_nodes;
     M.nt_norm = T.nt_norm;
     return BHN_OK;
 }
 
-}  // namespace synch
-}  // namespace bhn
-
-extern "C" int bhn_brick_precompute(const double *rho, const double *theta_e, const double *b_con, int64_t cells,
-                                    const bhn_synchrotron_model *m, void *coeffs, int32_t coeff_bytes, void *stream) {
-    using namespace bhn;
-    using namespace bhn::synch;
+// The launches behind the entry points: scratch as Scratch::p, or NULL.
+static int precompute(const double *rho, const double *theta_e, const double *b_con, int64_t cells,
+                      const bhn_synchrotron_model *m, void *coeffs, int32_t coeff_bytes, void *scratch,
+                      int64_t scratch_bytes, cudaStream_t s) {
     if (cells < 1) return fail(BHN_ERR_VALUE, "the snapshot must contain at least one cell");
     if (!rho || !theta_e || !b_con || !coeffs) return fail(BHN_ERR_VALUE, "missing snapshot or output buffer");
     if (coeff_bytes != 4 && coeff_bytes != 8) return fail(BHN_ERR_VALUE, "brick values must be float32 or float64");
     PrecomputeParams P;
-    void *tables = nullptr;
-    cudaStream_t s = as_stream(stream);
+    Scratch tables{scratch, scratch_bytes};
     int rc = build_model(m, cells, P.M, tables, s);
     if (rc) return rc;
     P.nu = m->nu_hz;
@@ -618,20 +628,16 @@ extern "C" int bhn_brick_precompute(const double *rho, const double *theta_e, co
     const int64_t batches = (cells + P.per_warp - 1) / P.per_warp;
     const int64_t blocks = std::min<int64_t>((batches + 3) / 4, (int64_t)sms * 16);
     precompute_kernel<<<(unsigned)blocks, 128, 0, s>>>(P);
-    const cudaError_t e = cudaGetLastError();
-    stream_free(tables, s);
-    return e == cudaSuccess ? BHN_OK : cuda_fail(e, "precompute_kernel");
+    BHN_LAUNCH_CHECK("precompute_kernel");
+    return BHN_OK;
 }
 
-extern "C" int bhn_synchrotron_coefficients(const double *frames, int64_t n, const bhn_synchrotron_model *m,
-                                            double *out, void *stream) {
-    using namespace bhn;
-    using namespace bhn::synch;
+static int frame_coefficients(const double *frames, int64_t n, const bhn_synchrotron_model *m, double *out,
+                              void *scratch, int64_t scratch_bytes, cudaStream_t s) {
     if (n < 1) return fail(BHN_ERR_VALUE, "at least one plasma frame is required");
     if (!frames || !out) return fail(BHN_ERR_VALUE, "missing frame or output buffer");
     FrameParams P;
-    void *tables = nullptr;
-    cudaStream_t s = as_stream(stream);
+    Scratch tables{scratch, scratch_bytes};
     int rc = build_model(m, n, P.M, tables, s);
     if (rc) return rc;
     P.nu = m->nu_hz;
@@ -643,7 +649,45 @@ extern "C" int bhn_synchrotron_coefficients(const double *frames, int64_t n, con
     const int64_t batches = (n + P.per_warp - 1) / P.per_warp;
     const int64_t blocks = std::min<int64_t>((batches + 3) / 4, (int64_t)sms * 16);
     frame_coefficients_kernel<<<(unsigned)blocks, 128, 0, s>>>(P);
-    const cudaError_t e = cudaGetLastError();
-    stream_free(tables, s);
-    return e == cudaSuccess ? BHN_OK : cuda_fail(e, "frame_coefficients_kernel");
+    BHN_LAUNCH_CHECK("frame_coefficients_kernel");
+    return BHN_OK;
 }
+
+}  // namespace synch
+}  // namespace bhn
+
+extern "C" {
+
+int64_t bhn_synchrotron_scratch_bytes(const bhn_synchrotron_model *m) {
+    std::lock_guard<std::mutex> g(bhn::synch::T_lock);
+    bhn::synch::Model M;
+    int64_t bytes = 0;
+    if (bhn::synch::plan_model(m, INT64_MAX, M, bytes)) return -1;  // the tables of many frames are the larger ones
+    return (bytes + 255) & ~(int64_t)255;
+}
+
+int bhn_brick_precompute(const double *rho, const double *theta_e, const double *b_con, int64_t cells,
+                         const bhn_synchrotron_model *m, void *coeffs, int32_t coeff_bytes, void *stream) {
+    return bhn::synch::precompute(rho, theta_e, b_con, cells, m, coeffs, coeff_bytes, nullptr, 0, bhn::as_stream(stream));
+}
+
+int bhn_brick_precompute_scratch(const double *rho, const double *theta_e, const double *b_con, int64_t cells,
+                                 const bhn_synchrotron_model *m, void *coeffs, int32_t coeff_bytes, void *scratch,
+                                 int64_t scratch_bytes, void *stream) {
+    if (!scratch) return bhn::fail(BHN_ERR_VALUE, "model scratch must not be NULL");
+    return bhn::synch::precompute(rho, theta_e, b_con, cells, m, coeffs, coeff_bytes, scratch, scratch_bytes,
+                                  bhn::as_stream(stream));
+}
+
+int bhn_synchrotron_coefficients(const double *frames, int64_t n, const bhn_synchrotron_model *m, double *out,
+                                 void *stream) {
+    return bhn::synch::frame_coefficients(frames, n, m, out, nullptr, 0, bhn::as_stream(stream));
+}
+
+int bhn_synchrotron_coefficients_scratch(const double *frames, int64_t n, const bhn_synchrotron_model *m, double *out,
+                                         void *scratch, int64_t scratch_bytes, void *stream) {
+    if (!scratch) return bhn::fail(BHN_ERR_VALUE, "model scratch must not be NULL");
+    return bhn::synch::frame_coefficients(frames, n, m, out, scratch, scratch_bytes, bhn::as_stream(stream));
+}
+
+}  // extern "C"

@@ -493,11 +493,25 @@ __device__ __forceinline__ void coefficients(TableSmem &S, const Model &M, const
     }
 }
 
-// Host: the device model for a C model, with its tables built on `stream` in a
-// stream-ordered allocation that `tables` names; the caller frees it there
-// (stream_free) after its last kernel.  `frames`: about how many frames the
-// tables will serve (from kGroupFrames on, the power law's nodes are grouped).
-int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &out, void *&tables, cudaStream_t stream);
+// The tables' memory: the caller's (p, bytes), or with p NULL a stream-ordered
+// allocation, freed on its stream after the owner's last kernel.
+struct Scratch {
+    void *p = nullptr;
+    int64_t bytes = 0;
+    bool owned = false;
+    cudaStream_t stream = nullptr;
+    Scratch(void *p_, int64_t bytes_) : p(p_), bytes(bytes_) {}
+    Scratch(const Scratch &) = delete;
+    ~Scratch() {
+        if (owned) stream_free(p, stream);
+    }
+};
+
+// Host: the device model for a C model, with its tables built on `stream` in
+// `tables`, which outlives the caller's kernels.  `frames`: about how many
+// frames the tables will serve (from kGroupFrames on, the power law's nodes are
+// grouped).
+int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &out, Scratch &tables, cudaStream_t stream);
 
 }  // namespace synch
 }  // namespace bhn

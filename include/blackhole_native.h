@@ -387,6 +387,20 @@ typedef struct bhn_synchrotron_model {
 int bhn_brick_precompute(const double *rho, const double *theta_e, const double *b_con, int64_t cells,
                          const bhn_synchrotron_model *model, void *coeffs, int32_t coeff_bytes, void *stream);
 
+/* Device memory of a model's tables.  bhn_brick_precompute,
+ * bhn_synchrotron_coefficients and bhn_grrt_render tabulate the model's sums
+ * once per call.  They take the tables' memory (5 MB for the Hybrid default,
+ * up to about 8.4) from a stream-ordered pool of the library's own, one
+ * per device, which keeps up to 64 MB between calls until the process ends;
+ * BHN_ERR_CUDA when the device has no memory left.  Their _scratch forms below
+ * allocate nothing: the caller passes bhn_synchrotron_scratch_bytes(model) bytes
+ * (-1 for a model that they refuse), 256-byte aligned, which may be reused
+ * once the call's work on its stream is done.  Same results. */
+int64_t bhn_synchrotron_scratch_bytes(const bhn_synchrotron_model *model);
+int bhn_brick_precompute_scratch(const double *rho, const double *theta_e, const double *b_con, int64_t cells,
+                                 const bhn_synchrotron_model *model, void *coeffs, int32_t coeff_bytes, void *scratch,
+                                 int64_t scratch_bytes, void *stream);
+
 /* The model's 11 coefficients for n local plasma frames, FP64 on the device.
  * Replaces ThermalSynchrotronCoefficients.coefficients,
  * NonthermalPowerLawSynchrotronCoefficients.coefficients and
@@ -398,6 +412,8 @@ int bhn_brick_precompute(const double *rho, const double *theta_e, const double 
  * models' own; the scaling fields of the model are not used. */
 int bhn_synchrotron_coefficients(const double *frames, int64_t n, const bhn_synchrotron_model *model, double *out,
                                  void *stream);
+int bhn_synchrotron_coefficients_scratch(const double *frames, int64_t n, const bhn_synchrotron_model *model,
+                                         double *out, void *scratch, int64_t scratch_bytes, void *stream);
 
 /* ---- physical polarized GRRT through a GRMHD snapshot --------------------------
  * Replaces polarized_renderer.render_stokes_image (python/blackhole_sim/
@@ -429,6 +445,12 @@ int bhn_grrt_render(const double *fields, const double *r_grid, int32_t nr, cons
                     const double *phi_grid, int32_t np, const bhn_view *view, const bhn_synchrotron_model *model,
                     const bhn_grrt_config *cfg, void *scratch, int64_t scratch_bytes, double *out, double *diag,
                     void *stream);
+/* The same with the model's tables in caller memory (bhn_synchrotron_scratch_bytes). */
+int bhn_grrt_render_scratch(const double *fields, const double *r_grid, int32_t nr, const double *theta_grid,
+                            int32_t nt, const double *phi_grid, int32_t np, const bhn_view *view,
+                            const bhn_synchrotron_model *model, const bhn_grrt_config *cfg, void *scratch,
+                            int64_t scratch_bytes, void *model_scratch, int64_t model_scratch_bytes, double *out,
+                            double *diag, void *stream);
 
 /* ---- the reference's brick renderer (RK4 fixed step) ----------------------
  * Replaces render_stokes_image_bricks / render_tile_stokes_bricks
