@@ -127,3 +127,17 @@ def test_grrt_pool_form_agrees():
         mp.setattr(grrt, "_declare", lambda: Pool)
         got = grrt.render_stokes_image_device(cfg, snap, scaling)
     assert calls == [1] and torch.equal(got.view(torch.int64), want.view(torch.int64))
+
+
+def test_sizes_do_not_depend_on_what_was_planned_before():
+    """Each pitch count's plan is kept; counts in any order, one component or two, give the sizes of a fresh process."""
+    models = [Hybrid(Thermal(pitch_nodes=a), Power(pitch_nodes=b)) for a in (64, 2, 16, 1) for b in (3, 64, 16)]
+    first = [_bytes(m) for m in models]
+    assert [_bytes(m) for m in reversed(models)] == first[::-1]
+    code = ("import blackhole_native as bn\nfrom blackhole_native import synchrotron as s\n"
+            "m = s.model_struct(bn.HybridSynchrotronCoefficients(bn.ThermalSynchrotronCoefficients(pitch_nodes=2),"
+            " bn.NonthermalPowerLawSynchrotronCoefficients(pitch_nodes=64)), 230e9, s._UNIT_SCALING)\n"
+            "print(s._table_bytes(s._table_values(m)))")
+    fresh = subprocess.run([sys.executable, "-c", code], env={**__import__("os").environ, "PYTHONPATH": str(PKG_ROOT)},
+                           capture_output=True, text=True, timeout=300)
+    assert int(fresh.stdout) == _bytes(Hybrid(Thermal(pitch_nodes=2), Power(pitch_nodes=64)))
