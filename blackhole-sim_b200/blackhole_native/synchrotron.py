@@ -115,7 +115,9 @@ class _DeviceCoefficients:
     def coefficients_batch(self, frames, nu_hz: float):
         """(n, 11) coefficients for n frames.  ``frames`` is an (n, 5) array or
         a list of frames (host: a numpy array is returned) or an (n, 5) float64
-        CUDA tensor (the result stays on the device)."""
+        CUDA tensor (the result stays on the device).  A frame's bits do not
+        depend on the frames beside it; batches of 8,192 frames and more sum the
+        power law's nodes in groups, which agrees with shorter ones to rounding."""
         on_device = isinstance(frames, torch.Tensor) and frames.is_cuda
         if on_device:
             if frames.dtype != torch.float64 or frames.dim() != 2 or frames.shape[1] != 5:

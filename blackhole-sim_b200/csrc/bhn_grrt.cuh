@@ -411,8 +411,8 @@ static int grrt_render(const double *fields, const double *r_grid, int32_t nr, c
     cudaStream_t s = as_stream(stream);
     CoefParams C;
     synch::Scratch tables(model_scratch, model_scratch_bytes);
-    // (a ray lists about a thousand segments; the same tables for every chunk, so the image does not depend on it)
-    int rc = synch::build_model(model, rays * 1000, C.M, tables, s);
+    // grouped for every size: a pixel must not depend on the crop or the chunk (a ray lists about a thousand segments)
+    int rc = synch::build_model(model, true, C.M, tables, s);
     if (rc) return rc;
     rc = bhn_render_prepare(view, 1, scratch, scratch_layout(1).total, stream);  // FP64 camera tables of the view
     if (rc) return rc;

@@ -482,14 +482,15 @@ void set_table(SumTable &T, const SumPlan &P, const double2 *rows) {
 }
 
 // Power-law nodes per row: 8 (28 rows of the default 224 nodes, one per lane)
-// while the group's sum has at most 64 terms and its span fits the cells, once
-// the frames repay its table (a call without and with groups: 5,000 Hybrid frames
+// while the group's sum has at most 64 terms and its span fits the cells.  Bakes
+// and images always take groups; frame batches from kGroupFrames on, where they
+// repay the group's table (a call without and with groups: 5,000 Hybrid frames
 // 53.6 and 59.6 us, 8,192 67.5 and 65.8; power law alone 4,000 38.6 and 41.2,
 // 8,192 47.5 and 43.5, 12,000 60.6 and 47.3).
 constexpr int64_t kGroupFrames = 8192;
-int group_size(const SumPlan &A, int gamma_n, double lr, int64_t frames) {
+int group_size(const SumPlan &A, int gamma_n, double lr, bool grouped) {
     int g = 1;
-    while (frames >= kGroupFrames && 2 * g * A.n <= 64 && 2 * g <= 8 && 2 * g <= gamma_n &&
+    while (grouped && 2 * g * A.n <= 64 && 2 * g <= 8 && 2 * g <= gamma_n &&
            cells_of(A.y0, A.shift_max + 2.0 * lr * (2 * g - 1)) <= kMaxCells)
         g *= 2;
     return g;
@@ -501,7 +502,7 @@ TableParams T;  // ~25 KB: kept off the host stack; filled and launched under th
 std::mutex T_lock;
 int64_t T_rows[3];  // rows of each sum's own table (0: off, or another sum's)
 int T_same[3];      // which table serves each sum
-int plan_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, int64_t &bytes) {
+int plan_model(const bhn_synchrotron_model *m, bool grouped, Model &M, int64_t &bytes) {
     if (!m) return fail(BHN_ERR_VALUE, "synchrotron model must not be NULL");
     if (!std::isfinite(m->nu_hz)) return fail(BHN_ERR_VALUE, "nu_hz must be finite");
     auto check_comp = [](int on, int gn, int pn) {
@@ -554,7 +555,7 @@ int plan_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, int64_t
         SumPlan &B = T.plan[1];
         T.nt_n = M.nt.gamma_n;
         const double lr = (std::log(M.nt.gamma_max) - std::log(M.nt.gamma_min)) / (T.nt_n - 1);
-        T.nt_group = group_size(A, T.nt_n, lr, frames);
+        T.nt_group = group_size(A, T.nt_n, lr, grouped);
         T.p = M.nt.p;
         T.gamma_min = M.nt.gamma_min;
         T.gamma_max = M.nt.gamma_max;
@@ -582,10 +583,10 @@ int plan_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, int64_t
 
 }  // namespace
 
-int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &M, Scratch &tables, cudaStream_t stream) {
+int build_model(const bhn_synchrotron_model *m, bool grouped, Model &M, Scratch &tables, cudaStream_t stream) {
     std::lock_guard<std::mutex> g(T_lock);
     int64_t bytes = 0;
-    int rc = plan_model(m, frames, M, bytes);
+    int rc = plan_model(m, grouped, M, bytes);
     if (rc || bytes == 0) return rc;
     if (!tables.p) {
         rc = stream_alloc(&tables.p, bytes, stream);
@@ -626,7 +627,7 @@ static int precompute(const double *rho, const double *theta_e, const double *b_
     if (coeff_bytes != 4 && coeff_bytes != 8) return fail(BHN_ERR_VALUE, "brick values must be float32 or float64");
     PrecomputeParams P;
     Scratch tables{scratch, scratch_bytes};
-    int rc = build_model(m, cells, P.M, tables, s);
+    int rc = build_model(m, true, P.M, tables, s);  // always: a brick's values must not depend on its slabs
     if (rc) return rc;
     P.nu = m->nu_hz;
     P.rho = rho;
@@ -650,7 +651,7 @@ static int frame_coefficients(const double *frames, int64_t n, const bhn_synchro
     if (!frames || !out) return fail(BHN_ERR_VALUE, "missing frame or output buffer");
     FrameParams P;
     Scratch tables{scratch, scratch_bytes};
-    int rc = build_model(m, n, P.M, tables, s);
+    int rc = build_model(m, n >= kGroupFrames, P.M, tables, s);
     if (rc) return rc;
     P.nu = m->nu_hz;
     P.frames = frames;
@@ -674,7 +675,7 @@ int64_t bhn_synchrotron_scratch_bytes(const bhn_synchrotron_model *m) {
     std::lock_guard<std::mutex> g(bhn::synch::T_lock);
     bhn::synch::Model M;
     int64_t bytes = 0;
-    if (bhn::synch::plan_model(m, INT64_MAX, M, bytes)) return -1;  // the tables of many frames are the larger ones
+    if (bhn::synch::plan_model(m, true, M, bytes)) return -1;  // the grouped tables are the larger ones
     return (bytes + 255) & ~(int64_t)255;
 }
 

@@ -23,8 +23,9 @@
 // consecutive ones are a sum of shifted A's with fixed weights, the same for
 // every such group: a second table of that kind, T(L) = sum_{i < G} rho^i
 // A(L - i h), takes them in one row (8 nodes: 28 rows instead of 224).
-// The tables depend on the model only; a call builds them on its stream
-// (sum_table_kernel) in a stream-ordered allocation.
+// The tables depend on the model, and on whether the call takes groups (bakes and
+// images always, frames from kGroupFrames on); a call builds them on its stream
+// (sum_table_kernel) in the caller's scratch or a stream-ordered allocation.
 //
 // One warp then evaluates a batch of frames: the per-frame scalars are
 // computed by one lane per frame, the frames' integrals one after the other
@@ -414,7 +415,8 @@ struct Frame {
 
 // The 11 coefficients of the model (synchrotron.py:248-325) for up to 32
 // frames, one per lane (lane < count).  Warp-collective; each lane gets its
-// frame's.  A frame's result does not depend on its lane or on the others.
+// frame's.  For one model and form of its tables, a frame's result does not depend
+// on its lane or on the others.
 __device__ __forceinline__ void coefficients(TableSmem &S, const Model &M, const Frame &f, int count,
                                              double out[11]) {
     constexpr unsigned kWarp = 0xffffffffu;
@@ -508,10 +510,10 @@ struct Scratch {
 };
 
 // Host: the device model for a C model, with its tables built on `stream` in
-// `tables`, which outlives the caller's kernels.  `frames`: about how many
-// frames the tables will serve (from kGroupFrames on, the power law's nodes are
-// grouped).
-int build_model(const bhn_synchrotron_model *m, int64_t frames, Model &out, Scratch &tables, cudaStream_t stream);
+// `tables`, which outlives the caller's kernels.  grouped: the power law's
+// nodes in groups where their sum fits (the same integrals to rounding, 2e-15
+// over 8,191 frames; calls whose results should agree in every bit choose alike).
+int build_model(const bhn_synchrotron_model *m, bool grouped, Model &out, Scratch &tables, cudaStream_t stream);
 
 }  // namespace synch
 }  // namespace bhn

@@ -409,7 +409,9 @@ int bhn_brick_precompute_scratch(const double *rho, const double *theta_e, const
  * frames[n][5] = (n_e_cm3, theta_e, b_gauss, cos_pitch_to_los, evpa_rad)
  * (device), out[n][11] in PolarizedCoefficients field order, which is
  * COEFF_NAMES order (device).  No nan_to_num, no Theta_e floor beyond the
- * models' own; the scaling fields of the model are not used. */
+ * models' own; the scaling fields of the model are not used.  A frame's bits
+ * do not depend on the frames beside it, but from n = 8192 on the power law's
+ * nodes are summed in groups: the same coefficients to rounding (1e-11). */
 int bhn_synchrotron_coefficients(const double *frames, int64_t n, const bhn_synchrotron_model *model, double *out,
                                  void *stream);
 int bhn_synchrotron_coefficients_scratch(const double *frames, int64_t n, const bhn_synchrotron_model *model,
