@@ -401,11 +401,14 @@ SamplePoints sample_points(const double *coeffs, const double *rg, int64_t nr, c
 
 int launch_samples(SamplePoints P, bool step, cudaStream_t s) {
     const int64_t resident = (int64_t)std::max(1, sm_count_current_device()) * kSampleBlocks;
-    // Points a warp takes at a time: 32, and while warps would be left without any, half as many down to 4: a batch's
-    // rounds of corners follow one another (32 points 11 rounds, 4 points 2).  64 points 8.7 -> 5.0 us, 3,000 7.8 ->
-    // 4.9, 18,944 8.2 -> 7.0, 50,000 9.5 -> 9.1 (70,000, at 16 points: 10.3 -> 10.9).
-    P.per_warp = 32;
-    while (!P.order && P.per_warp > 4 && P.n <= resident * (kSampleThreads / 32) * (P.per_warp / 2)) P.per_warp /= 2;
+    // Points a warp takes at a time: a batch's rounds of corners follow one another (32 points 11 rounds, 4 points 2), but
+    // every batch pays for its two phases of a lane per point.  Kernel us at either side of the lines (two points a
+    // resident warp, 6, 12, and 16 where the corners come from memory), a 64 x 33 x 60 brick, step: 64 points 4.6 at 4 a
+    // warp and 5.0 at 8; 12,000 6.4 and 5.9; 26,000 at 8 and 16 7.2 and 7.1, 34,000 8.2 and 7.5; 50,000 at 16 and 32 8.9
+    // and 9.0, 62,000 9.9 and 9.5, 70,000 10.7 and 9.7; a brick of 352 MB 62,000 10.5 and 11.2, 75,000 12.1 and 13.6.
+    const int64_t warps = resident * (kSampleThreads / 32);
+    const bool in_l2 = 88 * (int64_t)P.nr * P.nt * P.np <= 100'000'000;
+    P.per_warp = P.order ? 32 : P.n <= 2 * warps ? 4 : P.n <= 6 * warps ? 8 : P.n <= (in_l2 ? 12 : 16) * warps ? 16 : 32;
     const int64_t groups = (P.n + P.per_warp - 1) / P.per_warp;
     const int threads = (int)std::min<int64_t>(kSampleThreads, 32 * std::max<int64_t>(2, (groups + resident - 1) / resident));
     const int64_t blocks = std::min(resident, (32 * groups + threads - 1) / threads);

@@ -81,10 +81,10 @@ def _sampler(nr, nt, np_, n, seed):
 
 
 def test_samplers_of_different_sizes(hammer):
-    """About 51, 77, 97 and 155 KB a block: small sets, so that the threads spend their time in the calls."""
+    """About 51, 50, 59 and 124 KB a block: small sets, so that the threads spend their time in the calls."""
     L = _lib.lib()
-    sets = [_sampler(3900, 3, 90, 2960, 1), _sampler(16, 9, 12, 11_840, 2), _sampler(2000, 3, 90, 12_400, 3),
-            _sampler(3900, 3, 90, 18_944, 4)]
+    sets = [_sampler(3900, 3, 90, 2960, 1), _sampler(16, 9, 12, 60_000, 2), _sampler(2000, 3, 90, 12_400, 3),
+            _sampler(3900, 3, 90, 28_000, 4)]
     want = []
     for args, out, _ in sets:
         _lib.check(L.bhn_sample_brick_trilinear(*args, dev.stream_ptr()))
