@@ -131,8 +131,8 @@ constexpr int kSeries = 12;  // Taylor terms before economisation
 // Terms first, first + stride, ... of a row's Taylor series (F and G) about
 // its centre, in units of the half width h, each times its degree's factorial.  A term sees the table segment at
 // its x (numpy.interp: constant past either end of the knots).
-__host__ __device__ inline void row_series(const KernelTable &K, const SumPlan &P, double centre, double h, int first,
-                                           int stride, double aF[kSeries], double aG[kSeries]) {
+__device__ inline void row_series(const KernelTable &K, const SumPlan &P, double centre, double h, int first, int stride,
+                                  double aF[kSeries], double aG[kSeries]) {
     for (int d = 0; d < kSeries; ++d) aF[d] = aG[d] = 0.0;
     for (int t = first; t < P.n; t += stride) {
         const double x = centre - P.shift[t];
@@ -159,7 +159,7 @@ __host__ __device__ inline void row_series(const KernelTable &K, const SumPlan &
 
 // The series of row_series economised to degree 7 (v^n -> v^n - T_n(v) / 2^(n-1), n = 11 .. 8,
 // v = z / h) and scaled to powers of z.
-__host__ __device__ inline void row_coefficients(double a[kSeries], double h, double co[8]) {
+__device__ inline void row_coefficients(double a[kSeries], double h, double co[8]) {
     // Chebyshev polynomials T_11 .. T_8 below their leading terms
     const double t11[5] = {-11.0, 220.0, -1232.0, 2816.0, -2816.0};  // v, v^3 .. v^9
     const double t10[5] = {-1.0, 50.0, -400.0, 1120.0, -1280.0};     // 1, v^2 .. v^8
@@ -179,7 +179,7 @@ __host__ __device__ inline void row_coefficients(double a[kSeries], double h, do
 }
 
 // The row's cell, and its centre and half width in L.
-__host__ __device__ inline void row_place(const SumPlan &P, int row, double &centre, double &h) {
+__device__ inline void row_place(const SumPlan &P, int row, double &centre, double &h) {
     int c = 0, hi = P.cells;  // the cell whose first row is the last at or before `row`
     while (hi - c > 1) {
         const int mid = (c + hi) >> 1;

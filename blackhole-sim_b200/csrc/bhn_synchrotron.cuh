@@ -152,27 +152,14 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // 2^n, -1022 <= n <= 1023
-__host__ __device__ __forceinline__ double pow2(int n) {
-#ifdef __CUDA_ARCH__
-    return __hiloint2double((n + 1023) << 20, 0);
-#else
-    return std::ldexp(1.0, n);
-#endif
-}
+__device__ __forceinline__ double pow2(int n) { return __hiloint2double((n + 1023) << 20, 0); }
 
 // L at the centre of row `sub` of 2^split in the piece [left, left + width) of cell c (table build and lookup alike).
-__host__ __device__ __forceinline__ double row_centre(double y0, double delta, double c, double left, double width,
-                                                      int split, int sub) {
+__device__ __forceinline__ double row_centre(double y0, double delta, double c, double left, double width, int split,
+                                             int sub) {
     double at = 0.5;
     if (split) at = ((double)sub + 0.5) * pow2(-split);  // exact
     return fma(c + fma(at, width, left), delta, y0);
-}
-
-// numpy.geomspace(start, stop, n)[i] (logspace of a linspace; exact end points).
-__device__ __forceinline__ double geom_node(double start, double stop, double ls, double step, int i, int n) {
-    if (i <= 0) return start;
-    if (i >= n - 1) return stop;
-    return pow(10.0, __dadd_rn(__dmul_rn((double)i, step), ls));
 }
 
 // The row of L and L minus its centre.  The nearest cell comes from adding and
