@@ -646,7 +646,7 @@ PRECOMPUTE = dict(nr=256, ntheta=128, nphi=256, spin_a=0.9375, seed=5, nu_hz=230
 PRECOMPUTE_PROFILE = REPO / "profiles" / "precompute_kernel_snapshot_2M_cells.md"
 PRECOMPUTE_PROFILE_CELLS = 64 * 128 * 256   # the captured case; its traffic scales with the cells
 GRRT_SNAPSHOT = dict(nr=64, ntheta=32, nphi=64, spin_a=0.9375, seed=0)
-GRRT_PROFILE = REPO / "profiles" / "grrt_kernel_default_image.md"   # the snapshot is read once per launch
+GRRT_PROFILE = REPO / "profiles" / "grrt_kernel_default_image.md"   # all launches of the default image
 # calibration.PhysicalScaling of a 4.3e6 solar-mass hole at 8.3 kpc with code units rho 3e-18 g/cm^3, B 25 G
 SCALING = dict(mass_bh_g=8.54e39, distance_cm=2.57e22, rho_cgs_per_code=3.0e-18, b_gauss_per_code=25.0)
 
@@ -676,22 +676,26 @@ def fp64_peaks(device, stream) -> dict:
     return out
 
 
-def exps_per_evaluation(model_struct) -> int:
-    """Double exp() calls one coefficient evaluation needs: the thermal
-    weight of every Lorentz-factor node.  (The sums over the pitch angles come
-    from tables, built once a call: a row of 16 multiply-adds a node in place
-    of two exp() for each of its 8 distinct pitch angles, 6,656 in all for
-    the default model.)"""
-    return int(model_struct.thermal_gamma_n) if model_struct.thermal else 0
+# Warp instructions per unit of work of the present kernels (profiles/current_kernels.md): precompute_kernel per cell, and
+# the trace, coefficient and transfer kernels of a whole 160 x 90 image per emitting segment (1,781 of them coefficients).
+PRECOMPUTE_WARP_INST_PER_CELL = 1802
+GRRT_WARP_INST_PER_SEGMENT = 1866
 
 
-def exp_roofline(evals: float, seconds: float, peaks: dict, per_eval: int, kernel: str) -> dict:
-    achieved = evals * per_eval / seconds
-    return {"bound": "fp64", "achieved": round(achieved / 1e9, 2), "peak": round(peaks["exp_per_s"] / 1e9, 2),
-            "unit": "Gexp/s", "frac": round(achieved / peaks["exp_per_s"], 4), "traffic": None,
-            "peak_source": "measured in this run (bhn_fp64_peak_probe, 8 chains of x <- exp(-x) per thread)",
-            "kernel": kernel, "exp_per_unit": per_eval,
-            "fp64_fma_tflops_measured": round(peaks["fma_tflops"], 2)}
+def issue_roofline(units: float, seconds: float, inst_per_unit: int, clocks: dict | None, device, kernel: str) -> dict:
+    """Issue slots: no pipe of these kernels is half full and memory runs at a
+    few per cent, so the rate is warp instructions a second against one per
+    scheduler and clock (4 schedulers per SM)."""
+    import torch
+
+    mhz = (clocks or {}).get("sm_mhz") or 1965
+    peak = 4 * torch.cuda.get_device_properties(device).multi_processor_count * mhz * 1e6
+    achieved = units * inst_per_unit / seconds
+    return {"bound": "issue", "achieved": round(achieved / 1e9, 2), "peak": round(peak / 1e9, 2),
+            "unit": "G warp instructions/s", "frac": round(achieved / peak, 4), "traffic": None,
+            "peak_source": f"4 schedulers per SM at {mhz} MHz (the clock sampled in this run)",
+            "kernel": kernel, "warp_instructions_per_unit": inst_per_unit,
+            "instruction_source": "smsp__inst_executed.sum (profiles/current_kernels.md)"}
 
 
 def timed_launches(fn, k: int, stream, device) -> list[float]:
@@ -740,7 +744,6 @@ def bench_precompute(args) -> dict | None:
         _lib_check(L.bhn_brick_precompute(dev.ptr(d_rho), dev.ptr(d_te), dev.ptr(d_b), cells, ctypes.byref(m),
                                           dev.ptr(out), 4, stream.cuda_stream))
 
-    peaks = fp64_peaks(device, stream)
     for _ in range(args.warmup):
         launch()
     torch.cuda.synchronize(device)
@@ -788,7 +791,8 @@ def bench_precompute(args) -> dict | None:
                    "cells_per_step": cells, "l2": f"inputs larger than L2 ({cells * 48 / 1e6:.0f} MB of float64 fields)",
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
         "e2e": e2e, "gpu_launches": args.steps * 2, "clocks": clk,  # sum_table_kernel + precompute_kernel
-        "roofline": dict(exp_roofline(cells, per_mean * 1e-3, peaks, exps_per_evaluation(m), "precompute_kernel"),
+        "roofline": dict(issue_roofline(cells, per_mean * 1e-3, PRECOMPUTE_WARP_INST_PER_CELL, clk, device,
+                                        "precompute_kernel"),
                          traffic=_scaled_traffic(PRECOMPUTE_PROFILE, cells / PRECOMPUTE_PROFILE_CELLS)),
         "cpu_baseline": cpu,
         "kernel_ms": {"mean": per_mean, "min": min(per), "max": max(per)},
@@ -852,7 +856,6 @@ def bench_grrt(args) -> dict | None:
     d = diag.cpu().numpy()
     segments, steps = float(d[..., 1].sum()), float(d[..., 6].sum())
     out = torch.empty_like(img)
-    peaks = fp64_peaks(device, stream)
     for _ in range(args.warmup):
         grrt.render_stokes_image_device(cfg, ds, scaling, out=out)
     clocks = ClockSampler(_uuid(device)).start()
@@ -887,7 +890,6 @@ def bench_grrt(args) -> dict | None:
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         cpu = grrt_cpu_baseline(snap, scaling, cfg, args.cpu_seconds)
-    m = grrt.model_struct(grrt.HybridSynchrotronCoefficients(), cfg.transfer.observing_frequency_hz, scaling)
     chunk = grrt.default_chunk(pixels)
     # setup_views, sum_table and init kernels, then trace / coefficient / transfer rounds
     launches_per_image = 3 + 3 * (cfg.max_steps // chunk + 2)
@@ -904,10 +906,9 @@ def bench_grrt(args) -> dict | None:
                    "l2": "snapshot (11.5 MB) resident in L2; the work is per-segment arithmetic",
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
         "e2e": e2e, "gpu_launches": args.steps * launches_per_image, "clocks": clk,
-        "roofline": dict(exp_roofline(segments, per_mean * 1e-3, peaks, exps_per_evaluation(m),
-                                      "grrt_coef_kernel (timed: the whole render, all rounds of the trace, "
-                                      "coefficient and transfer kernels)"),
-                         traffic=profiled_traffic(GRRT_PROFILE)),
+        "roofline": dict(issue_roofline(segments, per_mean * 1e-3, GRRT_WARP_INST_PER_SEGMENT, clk, device,
+                                        "all rounds of grrt_trace_kernel, grrt_coef_kernel and grrt_transfer_kernel"),
+                         traffic=None if args.side else profiled_traffic(GRRT_PROFILE)),
         "cpu_baseline": cpu,
         "kernel_ms": {"mean": per_mean, "min": min(per), "max": max(per)},
     }
@@ -1108,10 +1109,11 @@ def bricks_cpu_baseline(grid, snap, cfg, target_s: float) -> dict:
 # The plugin's sample_and_step_stokes (native_kernels.py:325-407, lib.rs:308-366)
 MICRO = dict(nr=256, ntheta=128, nphi=256, points=1 << 24, seed=0, ds_cm=0.05, e2e_points=1 << 20)
 MICRO_PROFILE = REPO / "profiles" / "sample_and_step_kernel_16M_points.md"
-# Algorithmic bytes per point: the (r, theta, phi) triple, the 8 corner cells'
-# 11 float64 coefficients, the 4 float64 Stokes values written (the initial
-# vector is broadcast).
+# Bytes a point touches: the (r, theta, phi) triple, the 8 corner cells' 11 float64 coefficients and the 4 float64 Stokes
+# values written (the initial vector is broadcast).  Neighbouring points share corners, so what the call cannot do
+# without is the triple, the result and the brick once.
 MICRO_BYTES_PER_POINT = 3 * 8 + 8 * 11 * 8 + 4 * 8
+MICRO_OWN_BYTES_PER_POINT = 3 * 8 + 4 * 8
 
 
 def bench_micro(args) -> dict | None:
@@ -1208,7 +1210,8 @@ def bench_micro(args) -> dict | None:
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         cpu = micro_cpu_baseline(b, pts, M["ds_cm"], args.cpu_seconds)
     per_mean = statistics.mean(per)
-    achieved = MICRO_BYTES_PER_POINT * n / (per_mean * 1e-3) / 1e9
+    algorithmic = MICRO_OWN_BYTES_PER_POINT * n + b.coeffs.nbytes
+    achieved = algorithmic / (per_mean * 1e-3) / 1e9
     line = {
         "metric": "points/s", "value": value, "unit": "points/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": t_max / args.steps, "higher_is_better": True, "scaling": "weak",
@@ -1221,11 +1224,13 @@ def bench_micro(args) -> dict | None:
         # this package's kernels per step: cell keys + the ordered sampler (the radix sort's are the library's)
         "gpu_launches": args.steps * (3 if n >= kernels.SORT_MIN_POINTS else 1),
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                     "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": profiled_traffic(MICRO_PROFILE),
+                     "frac": round(achieved / peaks["hbm_gbs"], 4),
+                     "traffic": profiled_traffic(MICRO_PROFILE) if n == MICRO["points"] else None,
                      "peak_source": f"{peaks['source']} (MEASURED_PEAKS.json hbm_gbs)" if peaks["source"] == "measured"
                      else "fallback 6.65 TB/s",
                      "kernel": "sample_points_kernel<true, true> (timed: cell keys, radix sort and the ordered "
-                               "sampler)", "algorithmic_bytes_per_point": MICRO_BYTES_PER_POINT},
+                               "sampler)", "algorithmic_bytes_per_launch": algorithmic,
+                     "touched_bytes_per_point": MICRO_BYTES_PER_POINT},
         "cpu_baseline": cpu,
         "kernel_ms": {"mean": per_mean, "min": min(per), "max": max(per)},
         "stokes_rk2_brick": stokes_rk2,
