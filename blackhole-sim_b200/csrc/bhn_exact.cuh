@@ -64,17 +64,15 @@ struct AxisHints {
     double g0[3], gn[3];  // first and last knot
 };
 
-// A group of `stride` threads classifies an axis together: thread `first` takes every stride-th knot, most(x) is the
-// group's largest x.  NaN or unsorted knots classify as search, which is always exact.
-template <class Most>
-__device__ __forceinline__ void classify_axis(const double *g, int n, int first, int stride, Most most, int &kind,
-                                              double &off, double &inv) {
+__device__ __forceinline__ void classify_axis_warp(const double *g, int n, int lane, int &kind, double &off,
+                                                   double &inv) {
     kind = kSearch;
     off = inv = 0.0;
     const double d = (g[n - 1] - g[0]) / (n - 1);
     double dev = 0.0;
-    for (int k = first; k < n; k += stride) dev = fmax(dev, fabs(g[k] - (g[0] + k * d)));
-    if (most(dev) <= 0.25 * d) {
+    for (int k = lane; k < n; k += 32) dev = fmax(dev, fabs(g[k] - (g[0] + k * d)));
+    for (int o = 16; o > 0; o >>= 1) dev = fmax(dev, __shfl_xor_sync(0xffffffffu, dev, o));
+    if (dev <= 0.25 * d) {
         kind = kUniform;
         inv = 1.0 / d;
         off = g[0] * inv;
@@ -83,40 +81,37 @@ __device__ __forceinline__ void classify_axis(const double *g, int n, int first,
     if (!(g[0] > 0.0)) return;
     const double dl = log(g[n - 1] / g[0]) / (n - 1);
     double devl = 0.0;
-    for (int k = first; k < n; k += stride) devl = fmax(devl, fabs(log(g[k] / g[0]) - k * dl));
-    if (most(devl) <= 0.25 * dl) {
+    for (int k = lane; k < n; k += 32) devl = fmax(devl, fabs(log(g[k] / g[0]) - k * dl));
+    for (int o = 16; o > 0; o >>= 1) devl = fmax(devl, __shfl_xor_sync(0xffffffffu, devl, o));
+    if (devl <= 0.25 * dl) {
         kind = kGeometric;
         inv = 1.0 / dl;
         off = log(g[0]) * inv;
     }
 }
-__device__ __forceinline__ void set_axis_hint(AxisHints &h, int a, const double *g, int n, int kind, double off,
-                                              double inv) {
-    if (!(isfinite(off) && isfinite(inv)) || (a == 2 && kind == kGeometric)) kind = kSearch;  // phi's guess is the uniform one
-    h.kind[a] = kind;
-    h.off[a] = off;
-    h.inv[a] = inv;
-    h.g0[a] = g[0];
-    h.gn[a] = g[n - 1];
-}
-__device__ __forceinline__ double warp_max(double v) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 
 // Every thread of the block must call this (it synchronises the block); the
-// block needs at least one full warp.
+// block needs at least one full warp.  NaN or unsorted knots classify as
+// search, which is always exact.
 __device__ __forceinline__ void load_axis_hints(AxisHints &h, const double *rg, int nr, const double *tg, int nt,
                                                 const double *pg, int np) {
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         for (int a = 0; a < 3; ++a) {
-            const double *g = a == 0 ? rg : (a == 1 ? tg : pg);
-            const int n = a == 0 ? nr : (a == 1 ? nt : np);
             int kind;
             double off, inv;
-            classify_axis(g, n, lane, 32, warp_max, kind, off, inv);
-            if (lane == 0) set_axis_hint(h, a, g, n, kind, off, inv);
+            classify_axis_warp(a == 0 ? rg : (a == 1 ? tg : pg), a == 0 ? nr : (a == 1 ? nt : np), lane, kind, off,
+                               inv);
+            if (!(isfinite(off) && isfinite(inv)) || (a == 2 && kind == kGeometric)) kind = kSearch;  // phi's guess is the uniform one
+            if (lane == 0) {
+                const double *g = a == 0 ? rg : (a == 1 ? tg : pg);
+                const int n = a == 0 ? nr : (a == 1 ? nt : np);
+                h.kind[a] = kind;
+                h.off[a] = off;
+                h.inv[a] = inv;
+                h.g0[a] = g[0];
+                h.gn[a] = g[n - 1];
+            }
         }
     }
     __syncthreads();

@@ -68,12 +68,13 @@ __device__ __forceinline__ int cell_phi(const double *g, int n, double p) {
     return i < 0 ? n - 1 : i;
 }
 
-// The axes' first-guess parameters (load_axis_hints' rule), for the key kernel:
+// The axes' first-guess parameters for the key kernel: load_axis_hints' rule with
 // a block per axis.  An axis of more than kHintKnots knots is searched instead:
 // its classification, two passes with a logarithm per knot, would take longer
 // than the searches of the smallest ordered set save.  A call of 300,000 points
 // through a geometric axis of 2^12, 2^16 and 2^20 knots: 148, 191 and 372 us (one
-// warp for all axes of any length: 181, 964 and 13,864).
+// warp for all axes of any length: 181, 964 and 13,864).  (The warp's form as a
+// call of a shared one cost the brick renderer 40 us an image.)
 constexpr int kHintThreads = 1024, kHintKnots = 1 << 14;
 __global__ void __launch_bounds__(kHintThreads) axis_hints_kernel(const double *rg, int nr, const double *tg, int nt,
                                                                   const double *pg, int np, AxisHints *out) {
@@ -81,16 +82,42 @@ __global__ void __launch_bounds__(kHintThreads) axis_hints_kernel(const double *
     const double *g = a == 0 ? rg : (a == 1 ? tg : pg);
     __shared__ double part[kHintThreads / 32];
     auto block_max = [&](double v) {
-        v = warp_max(v);
+        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
         __syncthreads();  // the previous call's reads
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
         __syncthreads();
-        return warp_max(part[threadIdx.x & 31]);
+        v = part[threadIdx.x & 31];
+        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+        return v;
     };
     int kind = kSearch;
     double off = 0.0, inv = 0.0;
-    if (n <= kHintKnots) classify_axis(g, n, (int)threadIdx.x, kHintThreads, block_max, kind, off, inv);
-    if (threadIdx.x == 0) set_axis_hint(*out, a, g, n, kind, off, inv);
+    if (n <= kHintKnots) {
+        const double d = (g[n - 1] - g[0]) / (n - 1);
+        double dev = 0.0;
+        for (int k = threadIdx.x; k < n; k += kHintThreads) dev = fmax(dev, fabs(g[k] - (g[0] + k * d)));
+        if (block_max(dev) <= 0.25 * d) {
+            kind = kUniform;
+            inv = 1.0 / d;
+            off = g[0] * inv;
+        } else if (a < 2 && g[0] > 0.0) {
+            const double dl = log(g[n - 1] / g[0]) / (n - 1);
+            double devl = 0.0;
+            for (int k = threadIdx.x; k < n; k += kHintThreads) devl = fmax(devl, fabs(log(g[k] / g[0]) - k * dl));
+            if (block_max(devl) <= 0.25 * dl) {
+                kind = kGeometric;
+                inv = 1.0 / dl;
+                off = log(g[0]) * inv;
+            }
+        }
+    }
+    if (threadIdx.x == 0) {
+        out->kind[a] = isfinite(off) && isfinite(inv) ? kind : kSearch;
+        out->off[a] = off;
+        out->inv[a] = inv;
+        out->g0[a] = g[0];
+        out->gn[a] = g[n - 1];
+    }
 }
 
 // The cell (r0, theta0, phi0) a point samples from, as one index; points the
