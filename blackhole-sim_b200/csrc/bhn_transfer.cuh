@@ -19,9 +19,9 @@
 // with a vector in place of 16 (and a squaring per doubling) with a matrix.
 // 2,000,003 cells at ||K ds|| ~ 0.05: 262 -> 69 us, where the cells' 304 MB
 // take 47; beyond 4 the products outnumber the squarings.  A warp with norms on
-// both sides of 4 takes both forms: 2M random cells of norms 1 to 20 take 550 us,
-// 337 by squaring alone; neighbouring cells of a brick are mostly alike (sorted by
-// norm, 243 and 311).  Queueing each warp's cells by form brought the mixed case to
+// both sides of 4 takes both forms: 2M random cells of norms 0.3 to 5.4 take 549
+// us, 335 by squaring alone; neighbouring cells of a brick are mostly alike (sorted
+// by norm, 243 and 311).  Queueing each warp's cells by form brought the mixed case to
 // 343, and the votes and reloads cost every other brick 4 to 6 %.
 
 #pragma once
